@@ -148,7 +148,10 @@ nrcps_status nrcps_autotune(nrcps_context *ctx, nrcps_precision prec, int L, int
  * context's device under its current options (no counterpart in the
  * reference; it names the kernel behind a measurement): *kind (0..12, see
  * "fused.kind") and *cluster (CTAs per cluster); both -1 when no fused
- * variant serves the shape.  Tunes nothing. */
+ * variant serves the shape.  (13, 1) names the kernel that holds an orbital in
+ * one SM (FP32, L = 32): it runs where no variant is forced and the batch
+ * fills the device; smaller batches run the autotuned variant, with the same
+ * results.  Tunes nothing. */
 nrcps_status nrcps_fused_choice(nrcps_context *ctx, nrcps_precision prec, int L, int *kind, int *cluster);
 
 /* ----------------------------------------------------- host-side tables
