@@ -12,6 +12,8 @@
 //   det S_n(Psi) = det S_n(Q) * prod_{i <= n} R_ii.
 // The running sum of log R_ii per orbital is kept per configuration and the
 // measured determinants are rescaled by exp(sum_{i<=n} log R_ii).
+#include <cooperative_groups.h>
+
 #include "common.cuh"
 
 namespace nrcps {
@@ -19,7 +21,7 @@ namespace nrcps {
 bool gram_tc_supported(int N, long vol, int nconf);
 nrcps_status gram_tc(nrcps_context* ctx, const void* psi, int N, long vol, int nconf, double* G);
 
-// G[c][i][j] for i <= j (the upper triangle the Cholesky reads), one block
+// FP64 orbitals: G[c][i][j] for i <= j (the upper triangle the Cholesky reads), one block
 // per configuration reading its orbitals once: tiles of GT sites of all N
 // orbitals go through shared memory (rows padded by one element so that the
 // rows a warp reads fall in different banks); each thread accumulates 2 x 2
@@ -151,171 +153,263 @@ __global__ void __launch_bounds__(256) gram_tile_kernel(const void* __restrict__
 }
 
 // Per configuration: Cholesky G = R^H R (R upper), Rinv = R^{-1}, and
-// logR[c][i] += log R_ii.  One thread per configuration; G is overwritten
-// with Rinv.  A non-positive pivot marks the configuration with NaN in logR.
-// f32_apply: the orbitals are FP32 and Rinv will be applied rounded to FP32;
-// the leading-minor identity det S_n(Psi) = det S_n(Psi Rinv) / prod_{i<n}
-// Rinv_ii then holds for the ROUNDED diagonal, so logR accumulates
+// logR[c][i] += log R_ii; G is overwritten with Rinv.  A non-positive pivot
+// marks the configuration with NaN in logR (and leaves its G as far as it
+// got).  f32_apply: the orbitals are FP32 and Rinv will be applied rounded to
+// FP32; the leading-minor identity det S_n(Psi) = det S_n(Psi Rinv) /
+// prod_{i<n} Rinv_ii then holds for the ROUNDED diagonal, so logR accumulates
 // -log(float(Rinv_ii)) instead of log R_ii.
-__global__ void chol_inv_kernel(double* __restrict__ G, int N, int nconf, double* __restrict__ logR, int f32_apply) {
-  for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < nconf; c += gridDim.x * blockDim.x) {
-    double* g = G + 2L * c * N * N;
-    auto re = [&](int i, int j) -> double& { return g[2 * (i * N + j)]; };
-    auto im = [&](int i, int j) -> double& { return g[2 * (i * N + j) + 1]; };
-    // Cholesky in place, upper triangle: G = R^H R
-    bool ok = true;
-    for (int i = 0; i < N && ok; ++i) {
-      double d = re(i, i);
-      for (int k = 0; k < i; ++k) d -= re(k, i) * re(k, i) + im(k, i) * im(k, i);
-      if (!(d > 0.0)) {
-        ok = false;
-        break;
-      }
-      const double rii = sqrt(d);
-      re(i, i) = rii;
-      im(i, i) = 0.0;
-      for (int j = i + 1; j < N; ++j) {
-        // R_ij = (G_ij - sum_k conj(R_ki) R_kj) / R_ii
-        double sr = re(i, j), si = im(i, j);
-        for (int k = 0; k < i; ++k) {
-          const double ar = re(k, i), ai = -im(k, i), br = re(k, j), bi = im(k, j);
-          sr -= ar * br - ai * bi;
-          si -= ar * bi + ai * br;
-        }
-        re(i, j) = sr / rii;
-        im(i, j) = si / rii;
-      }
+//
+// One block per configuration, the matrix in shared memory: the columns below
+// a pivot are updated by all threads at once, every entry in the order of the
+// sum over k (right-looking; the values a left-looking factorisation has), and
+// each row of the inverse by one thread per column.  A serial chain of N
+// square roots and divisions is left: 29 us for 256 matrices of N = 19, 34 us
+// for 1024 (one thread per matrix: 610 and 675 us).
+constexpr int CHOL_THREADS = 128;
+__global__ void __launch_bounds__(CHOL_THREADS) chol_inv_kernel(double* __restrict__ G, int N,
+                                                                double* __restrict__ logR, int f32_apply) {
+  extern __shared__ double2 cm[];  // [N][N]
+  const long c = blockIdx.x;
+  double2* g = reinterpret_cast<double2*>(G) + c * N * N;
+  for (int e = threadIdx.x; e < N * N; e += CHOL_THREADS)
+    if (e / N <= e % N) cm[e] = g[e];
+  __syncthreads();
+  bool ok = true;
+  for (int k = 0; k < N; ++k) {
+    const double d = cm[k * N + k].x;
+    if (!(d > 0.0)) {  // (the same for every thread)
+      ok = false;
+      break;
     }
-    if (!ok) {
-      for (int i = 0; i < N; ++i) logR[(long)c * N + i] = nan("");
-      continue;
+    const double rkk = sqrt(d);
+    __syncthreads();  // every thread has read the pivot
+    for (int j = k + threadIdx.x; j < N; j += CHOL_THREADS) {
+      if (j == k) cm[k * N + k] = make_double2(rkk, 0.0);
+      else cm[k * N + j] = make_double2(cm[k * N + j].x / rkk, cm[k * N + j].y / rkk);
     }
-    if (!f32_apply)
-      for (int i = 0; i < N; ++i) logR[(long)c * N + i] += log(re(i, i));
-    // Rinv (upper triangular) by back substitution, column by column, into
-    // the lower-left (unused) storage is not possible for complex R; invert
-    // in place row by row from the bottom: Rinv_ii = 1/R_ii,
-    // Rinv_ij = -(sum_{k=i+1..j} R_ik Rinv_kj) / R_ii for j > i.
-    for (int i = N - 1; i >= 0; --i) {
-      const double rii = re(i, i);
-      for (int j = N - 1; j > i; --j) {
-        double sr = 0, si = 0;
-        for (int k = i + 1; k <= j; ++k) {
-          const double ar = re(i, k), ai = im(i, k), br = re(k, j), bi = im(k, j);
-          sr += ar * br - ai * bi;
-          si += ar * bi + ai * br;
-        }
-        re(i, j) = -sr / rii;
-        im(i, j) = -si / rii;
+    __syncthreads();
+    // G_ij -= conj(R_ki) R_kj for k < i <= j
+    const int m = N - k - 1;
+    for (int e = threadIdx.x; e < m * m; e += CHOL_THREADS) {
+      const int i = k + 1 + e / m, j = k + 1 + e % m;
+      if (i > j) continue;
+      const double2 a = cm[k * N + i], b = cm[k * N + j];
+      double2 v = cm[i * N + j];
+      if (i == j) {
+        v.x -= a.x * a.x + a.y * a.y;
+      } else {
+        v.x -= a.x * b.x + a.y * b.y;
+        v.y -= a.x * b.y - a.y * b.x;
       }
-      re(i, i) = 1.0 / rii;
+      cm[i * N + j] = v;
     }
-    if (f32_apply)
-      for (int i = 0; i < N; ++i) logR[(long)c * N + i] -= log((double)(float)re(i, i));
+    __syncthreads();
   }
+  if (!ok) {
+    for (int e = threadIdx.x; e < N * N; e += CHOL_THREADS)
+      if (e / N <= e % N) g[e] = cm[e];
+    for (int i = threadIdx.x; i < N; i += CHOL_THREADS) logR[c * N + i] = nan("");
+    return;
+  }
+  if (!f32_apply)
+    for (int i = threadIdx.x; i < N; i += CHOL_THREADS) logR[c * N + i] += log(cm[i * N + i].x);
+  __syncthreads();
+  // Rinv in place, row by row from the bottom: Rinv_ii = 1 / R_ii,
+  // Rinv_ij = -(sum_{k=i+1..j} R_ik Rinv_kj) / R_ii for j > i (a thread per j;
+  // N <= 64 < CHOL_THREADS)
+  for (int i = N - 1; i >= 0; --i) {
+    const double rii = cm[i * N + i].x;
+    const int j = i + 1 + threadIdx.x;
+    double sr = 0, si = 0;
+    if (j < N)
+      for (int k = i + 1; k <= j; ++k) {
+        const double2 a = cm[i * N + k], b = cm[k * N + j];
+        sr += a.x * b.x - a.y * b.y;
+        si += a.x * b.y + a.y * b.x;
+      }
+    __syncthreads();  // row i has been read
+    if (j < N) cm[i * N + j] = make_double2(-sr / rii, -si / rii);
+    if (threadIdx.x == 0) cm[i * N + i] = make_double2(1.0 / rii, 0.0);
+    __syncthreads();
+  }
+  if (f32_apply)
+    for (int i = threadIdx.x; i < N; i += CHOL_THREADS) logR[c * N + i] -= log((double)(float)cm[i * N + i].x);
+  for (int e = threadIdx.x; e < N * N; e += CHOL_THREADS)
+    if (e / N <= e % N) g[e] = cm[e];
 }
 
-// Register-blocked variant for FP32 orbitals and N <= 20: thread (pair, g)
-// accumulates one 4 x 4 block (rows 4 bi.., columns 4 bj.., bi <= bj) of G
-// over the sites g, g + NG, .. of every tile -- 8 shared-memory loads per 64
-// FMAs instead of 4 per 16, as packed FP32x2 FMAs -- in FP32 over 32 sites
-// (4 tiles), then in FP64;
-// the NG = 16 site groups of a pair (16 adjacent lanes of one warp) are
-// summed by shuffles in FP64 at the end.
-// Tile rows N .. 19 are zero, so partial blocks need no special case.
-constexpr int G4_ROWS = 20;  // 5 row blocks of 4
-constexpr int G4_NG = 16;    // site groups per block pair
-__global__ void __launch_bounds__(256, 2) gram4_kernel(const void* __restrict__ psi, int N, long vol,
-                                                  double* __restrict__ G) {
+// FP32 orbitals.  One cluster of CTAs per configuration (and group of 16 block
+// pairs), each CTA a share of the sites; thread (slot, l) accumulates one
+// 4 x 4 block (rows 4 bi.., columns 4 bj.., bi <= bj) of G.  A stage of sites
+// goes from HBM through registers (the next stage's loads are in flight during
+// this one's products) into shared memory with real and imaginary parts apart,
+// so that a packed FP32x2 operand is the same part of two neighbouring sites:
+// 16 eight-byte loads feed 64 packed FMAs and no register is copied into a
+// pair.  Every FP32 sum runs over 32 sites, then goes into FP64 sums, which
+// wait in shared memory (32 per thread: in registers they would take the
+// place of the FP32 block).  Lanes, groups and CTAs are summed in a fixed
+// order; the split depends on the volume alone, so a configuration's G does
+// not depend on the batch it is in.
+// Bounds at N = 19, L = 32, 1024 configurations: one read of the orbitals 0.78
+// ms, the FMA pipe 1.2 ms (960 FMAs per site), the shared-memory loads about
+// the same.  Measured 2.61 ms (FMA pipe 45 %: the loads of a block and its
+// FMAs overlap in part only at 16 warps per SM); 3.07 ms with the (re, im)
+// pair of one site as the packed operand, which copies registers into pairs.
+// The split over a cluster serves small batches: 256 configurations 0.70 ms
+// against 0.90 (one CTA per configuration leaves 40 SMs half empty), N = 24,
+// 64 configurations at L = 24, whole call: 0.27 against 1.84.
+constexpr int G4_THREADS = 256;
+constexpr int G4_LANES = 16;                       // site lanes per slot
+constexpr int G4_SLOTS = G4_THREADS / G4_LANES;    // block pairs in flight
+constexpr int G4_FLUSH = 32;                       // sites per FP32 sum
+// sites per stage: small N leave slots free, which then share the stage's
+// sites (G groups per block pair)
+constexpr int g4_sites(int nb) { return nb == 1 ? 512 : nb <= 5 ? 128 : 64; }
+constexpr int g4_groups(int nb) { return nb == 1 ? 16 : nb == 2 ? 4 : nb == 3 ? 2 : 1; }
+constexpr int g4_chunks(int nb) { return (4 * nb * g4_sites(nb) / 2 + G4_THREADS - 1) / G4_THREADS; }
+constexpr size_t g4_smem(int nb) {
+  return sizeof(float) * 2 * 2 * 4 * nb * g4_sites(nb) + sizeof(double) * 32 * G4_THREADS;
+}
+
+template <int nb>  // blocks of four rows
+__global__ void __launch_bounds__(G4_THREADS, 2) gram4_kernel(const float2* __restrict__ psi, int N, long vol,
+                                                              int aligned, double* __restrict__ G) {
   extern __shared__ __align__(16) unsigned char gsm[];
-  float2* tiles = reinterpret_cast<float2*>(gsm);  // [2][G4_ROWS][GT + 1]
-  constexpr int TS = G4_ROWS * (GT + 1);
-  const long c = blockIdx.x;
-  const float2* base = reinterpret_cast<const float2*>(psi) + (size_t)c * N * vol;
-  const int nb = (N + 3) / 4, npairs = nb * (nb + 1) / 2;
-  const int g = threadIdx.x % G4_NG, pair = threadIdx.x / G4_NG;
-  const bool active = pair < npairs;
-  int bi = 0, rem = active ? pair : 0;
+  namespace cg = cooperative_groups;
+  cg::cluster_group cluster = cg::this_cluster();
+  const int split = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
+  const long c = blockIdx.x / split;
+  constexpr int npairs = nb * (nb + 1) / 2, rows = 4 * nb, T = g4_sites(nb), groups = g4_groups(nb);
+  constexpr int NCH = g4_chunks(nb);  // two-site pieces of a stage per thread
+  double* acc = reinterpret_cast<double*>(gsm);  // [32][G4_THREADS]
+  float* tiles = reinterpret_cast<float*>(acc + 32 * G4_THREADS);  // [2][re, im][rows][T]
+  constexpr int plane = rows * T, halfT = T / 2;
+  const float2* base = psi + (size_t)c * N * vol;
+  const int l = threadIdx.x % G4_LANES, slot = threadIdx.x / G4_LANES;
+  const int first = (int)blockIdx.y * G4_SLOTS;
+  const int here = npairs - first < G4_SLOTS ? npairs - first : G4_SLOTS;  // pairs of this CTA
+  const int grp = slot / here;
+  const bool active = grp < groups;
+  int bi = 0, rem = active ? first + slot % here : 0;
   while (rem >= nb - bi) {
     rem -= nb - bi;
     ++bi;
   }
   const int bj = bi + rem;
-  for (int e = threadIdx.x; e < 2 * (G4_ROWS - N) * (GT + 1); e += blockDim.x) {  // zero rows N..
-    const int b = e / ((G4_ROWS - N) * (GT + 1)), r = e % ((G4_ROWS - N) * (GT + 1));
-    tiles[b * TS + N * (GT + 1) + r] = make_float2(0.f, 0.f);
-  }
-  auto fill = [&](long p0, float2* t) {
-    const int ts = (int)((vol - p0) < GT ? (vol - p0) : GT);
-    for (int e = threadIdx.x; e < N * GT; e += blockDim.x) {
-      const int i = e / GT, q = e - i * GT;
-      if (q >= ts) t[i * (GT + 1) + q] = make_float2(0.f, 0.f);
-      else cp_async_elem(t + i * (GT + 1) + q, base + (size_t)i * vol + p0 + q, 8);
+#pragma unroll
+  for (int k = 0; k < 32; ++k) acc[k * G4_THREADS + threadIdx.x] = 0.0;
+  // this CTA's stages
+  const long stages = (vol + T - 1) / T;
+  const long s0 = stages * rank / split, s1 = stages * (rank + 1) / split;
+  // piece e of a stage: sites 2 j, 2 j + 1 of row i
+  float4 pre[NCH];
+  auto load = [&](long st) {
+#pragma unroll
+    for (int u = 0; u < NCH; ++u) {
+      const int e = threadIdx.x + u * G4_THREADS, i = e / halfT;
+      const long p = st * T + 2 * (e - i * halfT);
+      pre[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (i < N) {
+        const float2* q = base + (size_t)i * vol + p;
+        if (aligned && p + 1 < vol) {
+          pre[u] = __ldcs(reinterpret_cast<const float4*>(q));
+        } else {
+          if (p < vol) pre[u].x = q[0].x, pre[u].y = q[0].y;
+          if (p + 1 < vol) pre[u].z = q[1].x, pre[u].w = q[1].y;
+        }
+      }
     }
-    asm volatile("cp.async.commit_group;" ::: "memory");
   };
-  // FP32 partial sums over 4 tiles (32 sites per thread), then FP64
-  double acc[32];
-  float2 s[16];  // (re, im) of the 4 x 4 block, FP32 over 4 tiles
+  auto store = [&](float* t) {
 #pragma unroll
-  for (int k = 0; k < 32; ++k) acc[k] = 0.0;
+    for (int u = 0; u < NCH; ++u) {
+      const int e = threadIdx.x + u * G4_THREADS;
+      if (e < rows * halfT) {
+        reinterpret_cast<float2*>(t)[e] = make_float2(pre[u].x, pre[u].z);
+        reinterpret_cast<float2*>(t + plane)[e] = make_float2(pre[u].y, pre[u].w);
+      }
+    }
+  };
+  float2 sr[16], si[16];
 #pragma unroll
-  for (int k = 0; k < 16; ++k) s[k] = make_float2(0.f, 0.f);
-  fill(0, tiles);
-  int buf = 0, ntile = 0;
-  for (long p0 = 0; p0 < vol; p0 += GT, buf ^= 1, ++ntile) {
-    const float2* tile = tiles + buf * TS;
-    __syncthreads();  // every thread is done with the tile the next copies overwrite
-    if (p0 + GT < vol) fill(p0 + GT, tiles + (buf ^ 1) * TS);
-    else asm volatile("cp.async.commit_group;" ::: "memory");
-    asm volatile("cp.async.wait_group 1;" ::: "memory");
+  for (int k = 0; k < 16; ++k) sr[k] = si[k] = make_float2(0.f, 0.f);
+  int summed = 0;
+  auto flush = [&]() {
+#pragma unroll
+    for (int k = 0; k < 16; ++k) {
+      double* d = acc + 2 * k * G4_THREADS + threadIdx.x;
+      d[0] += (double)sr[k].x + (double)sr[k].y;
+      d[G4_THREADS] += (double)si[k].x + (double)si[k].y;
+      sr[k] = si[k] = make_float2(0.f, 0.f);
+    }
+    summed = 0;
+  };
+  if (s0 < s1) load(s0);
+  int buf = 0;
+  for (long st = s0; st < s1; ++st, buf ^= 1) {
+    float* t = tiles + buf * 2 * plane;
+    store(t);
+    if (st + 1 < s1) load(st + 1);
+    // (a thread stores into this buffer again only after the next stage's
+    // barrier, which every reader of this stage has then reached)
     __syncthreads();
     if (active) {
-      const float2* ta = tile + 4 * bi * (GT + 1) + g;
-      const float2* tb = tile + 4 * bj * (GT + 1) + g;
+      for (int ch = grp; ch < T / 32; ch += groups) {
+        const float* ta = t + 4 * bi * T + 32 * ch + 2 * l;
+        const float* tb = t + 4 * bj * T + 32 * ch + 2 * l;
+        float2 br[4], bm[4];
 #pragma unroll
-      for (int k = 0; k < GT / G4_NG; ++k) {
-        float2 a[4], b[4], bn[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          a[u] = ta[u * (GT + 1) + G4_NG * k];
-          b[u] = tb[u * (GT + 1) + G4_NG * k];
-          bn[u] = make_float2(b[u].y, -b[u].x);
+        for (int v = 0; v < 4; ++v) {
+          br[v] = *reinterpret_cast<const float2*>(tb + v * T);
+          bm[v] = *reinterpret_cast<const float2*>(tb + plane + v * T);
         }
-        // conj(a_u) b_v = (a.x b.x + a.y b.y, a.x b.y - a.y b.x): two packed FMAs
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
-          const float2 ax = make_float2(a[u].x, a[u].x), ay = make_float2(a[u].y, a[u].y);
+          const float2 ar = *reinterpret_cast<const float2*>(ta + u * T);
+          const float2 am = *reinterpret_cast<const float2*>(ta + plane + u * T);
+          const float2 nm = make_float2(-am.x, -am.y);
+          // conj(a) b = (ar br + am bm) + i (ar bm - am br)
 #pragma unroll
           for (int v = 0; v < 4; ++v) {
-            s[4 * u + v] = __ffma2_rn(ax, b[v], s[4 * u + v]);
-            s[4 * u + v] = __ffma2_rn(ay, bn[v], s[4 * u + v]);
+            sr[4 * u + v] = __ffma2_rn(ar, br[v], sr[4 * u + v]);
+            si[4 * u + v] = __ffma2_rn(ar, bm[v], si[4 * u + v]);
+          }
+#pragma unroll
+          for (int v = 0; v < 4; ++v) {
+            sr[4 * u + v] = __ffma2_rn(am, bm[v], sr[4 * u + v]);
+            si[4 * u + v] = __ffma2_rn(nm, br[v], si[4 * u + v]);
           }
         }
-      }
-      if ((ntile & 3) == 3 || p0 + GT >= vol) {
-#pragma unroll
-        for (int k = 0; k < 16; ++k) {
-          acc[2 * k] += (double)s[k].x;
-          acc[2 * k + 1] += (double)s[k].y;
-          s[k] = make_float2(0.f, 0.f);
-        }
+        if (++summed == G4_FLUSH) flush();
       }
     }
   }
-  // sum the 16 site groups of a pair (adjacent lanes) and write the upper triangle
-#pragma unroll
-  for (int k = 0; k < 32; ++k)
-    for (int o = G4_NG / 2; o > 0; o >>= 1) acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], o);
-  if (active && g == 0)
-    for (int u = 0; u < 4; ++u)
-      for (int v = 0; v < 4; ++v) {
-        const int i = 4 * bi + u, j = 4 * bj + v;
-        if (i >= N || j >= N || i > j) continue;
-        double* out = G + 2 * ((c * N + i) * (long)N + j);
-        out[0] = acc[2 * (4 * u + v)];
-        out[1] = acc[2 * (4 * u + v) + 1];
-      }
+  flush();
+  __syncthreads();
+  // the lanes and groups of every pair, then the cluster's CTAs
+  double* red = reinterpret_cast<double*>(tiles);  // [here][32], over the stages
+  for (int e = threadIdx.x; e < here * 32; e += G4_THREADS) {
+    const int pr = e / 32, k = e % 32;
+    double v = 0.0;
+    for (int g = 0; g < groups; ++g)
+      for (int j = 0; j < G4_LANES; ++j) v += acc[k * G4_THREADS + (g * here + pr) * G4_LANES + j];
+    red[e] = v;
+  }
+  cluster.sync();
+  // entries spread over the CTAs
+  for (int e = rank * G4_THREADS + threadIdx.x; e < here * 32; e += split * G4_THREADS) {
+    double v = 0.0;
+    for (int r = 0; r < split; ++r) v += cluster.map_shared_rank(red, r)[e];
+    int x = 0, y = first + e / 32;
+    while (y >= nb - x) {
+      y -= nb - x;
+      ++x;
+    }
+    const int k = (e % 32) / 2, i = 4 * x + k / 4, j = 4 * (x + y) + k % 4;
+    if (i < N && j < N && i <= j) G[2 * ((c * N + i) * (long)N + j) + (e & 1)] = v;
+  }
+  cluster.sync();  // peers keep their shared memory until every sum is read
 }
 
 // psi_{c,t}(p) <- sum_{i <= t} psi_{c,i}(p) Rinv[i][t]; one thread per site,
@@ -388,6 +482,49 @@ __global__ void __launch_bounds__(256) apply_rinv_kernel(void* __restrict__ psi,
   }
 }
 
+// The same for FP32 orbitals and N <= 24, two neighbouring sites per thread:
+// 16-byte loads and stores, and each entry of R^-1 read from shared memory
+// serves four packed FMAs.  Bound by HBM (one read, one write): 1024
+// configurations of N = 19 at L = 32 take 2.15 ms, 4.75 TB/s, 0.73 of a copy
+// (one site per thread: 2.27 ms).
+template <int NMAX>
+__global__ void __launch_bounds__(128) apply_rinv2_kernel(float2* __restrict__ psi, int N, long vol,
+                                                          const double* __restrict__ Rinv) {
+  __shared__ float4 r4[NMAX * NMAX];  // (re, re, im, im)
+  const long blocks_per_conf = (vol / 2 + 127) / 128;
+  const long c = blockIdx.x / blocks_per_conf;
+  const long p = 2 * ((blockIdx.x % blocks_per_conf) * 128 + threadIdx.x);
+  const bool live = p < vol;
+  float2* base = psi + (size_t)c * N * vol + (live ? p : 0);
+  float4 x[NMAX];
+#pragma unroll
+  for (int i = 0; i < NMAX; ++i)
+    if (i < N && live) x[i] = *reinterpret_cast<const float4*>(base + (size_t)i * vol);
+  for (int e = threadIdx.x; e < N * N; e += 128) {
+    const float ar = (float)Rinv[2L * (c * N * N + e)], ai = (float)Rinv[2L * (c * N * N + e) + 1];
+    r4[e] = make_float4(ar, ar, ai, ai);
+  }
+  __syncthreads();
+  if (!live) return;
+#pragma unroll
+  for (int t = NMAX - 1; t >= 0; --t) {
+    if (t >= N) continue;
+    float2 s0 = make_float2(0.f, 0.f), u0 = s0, s1 = s0, u1 = s0;
+#pragma unroll
+    for (int i = 0; i <= t; ++i) {
+      const float4 r = r4[i * N + t];
+      const float2 rr = make_float2(r.x, r.y), ri = make_float2(r.z, r.w);
+      const float2 x0 = make_float2(x[i].x, x[i].y), x1 = make_float2(x[i].z, x[i].w);
+      s0 = __ffma2_rn(x0, rr, s0);
+      u0 = __ffma2_rn(x0, ri, u0);
+      s1 = __ffma2_rn(x1, rr, s1);
+      u1 = __ffma2_rn(x1, ri, u1);
+    }
+    *reinterpret_cast<float4*>(base + (size_t)t * vol) =
+        make_float4(s0.x - u0.y, s0.y + u0.x, s1.x - u1.y, s1.y + u1.x);
+  }
+}
+
 // The determinants measured at slice t on the re-orthonormalised orbitals
 // Q = Psi R^-1, turned into those of Psi, with S_n = sum_{i<=n} log R_ii:
 //  mode 0 (SlaterDet::Run, S = <src|Psi> = <src|Q> R):
@@ -426,14 +563,63 @@ __global__ void rescale_dets_kernel(double* dets, const double* logR, int N, int
 template <int NMAX>
 static nrcps_status launch_apply(nrcps_context* ctx, void* psi, int N, long vol, int nconf, nrcps_precision prec,
                                  const double* Rinv) {
+  if constexpr (NMAX <= 24) {
+    if (prec == NRCPS_F32 && vol % 2 == 0 && (reinterpret_cast<uintptr_t>(psi) & 15) == 0) {
+      apply_rinv2_kernel<NMAX><<<(unsigned)((vol / 2 + 127) / 128 * nconf), 128, 0, ctx->stream>>>(
+          reinterpret_cast<float2*>(psi), N, vol, Rinv);
+      ctx->launches++;
+      return check_launch(ctx, "apply_rinv2_kernel");
+    }
+  }
   const long bpc = (vol + 255) / 256;
   const size_t sh = sizeof(double) * 2 * N * N;
+  if (sh > 48 * 1024) {
+    const void* kern = prec == NRCPS_F64 ? (const void*)apply_rinv_kernel<double, NMAX>
+                                         : (const void*)apply_rinv_kernel<float, NMAX>;
+    NRCPS_TRY(check_cuda(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh),
+                         "apply_rinv_kernel: smem attribute"));
+  }
   if (prec == NRCPS_F64)
     apply_rinv_kernel<double, NMAX><<<(unsigned)(bpc * nconf), 256, sh, ctx->stream>>>(psi, N, vol, nconf, Rinv);
   else
     apply_rinv_kernel<float, NMAX><<<(unsigned)(bpc * nconf), 256, sh, ctx->stream>>>(psi, N, vol, nconf, Rinv);
   ctx->launches++;
   return check_launch(ctx, "apply_rinv_kernel");
+}
+
+static nrcps_status launch_gram4(nrcps_context* ctx, const void* psi, int N, long vol, int nconf, double* G) {
+  const int nb = (N + 3) / 4, npairs = nb * (nb + 1) / 2;
+  const size_t sh = g4_smem(nb);
+  void (*kern)(const float2*, int, long, int, double*) = nullptr;
+  switch (nb) {
+#define NRCPS_CASE(B) \
+  case B:             \
+    kern = gram4_kernel<B>; \
+    break;
+    NRCPS_CASE(1) NRCPS_CASE(2) NRCPS_CASE(3) NRCPS_CASE(4) NRCPS_CASE(5) NRCPS_CASE(6) NRCPS_CASE(7) NRCPS_CASE(8)
+    NRCPS_CASE(9) NRCPS_CASE(10) NRCPS_CASE(11) NRCPS_CASE(12) NRCPS_CASE(13) NRCPS_CASE(14) NRCPS_CASE(15)
+    NRCPS_CASE(16)
+#undef NRCPS_CASE
+  }
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh);
+  if (e != cudaSuccess) return check_cuda(ctx, e, "gram4: smem attribute");
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  // CTAs per configuration: at least 16 stages each
+  const long stages = vol / g4_sites(nb);
+  attr[0].val.clusterDim.x = stages >= 128 ? 8 : stages >= 64 ? 4 : stages >= 32 ? 2 : 1;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cfg.gridDim = dim3((unsigned)nconf * attr[0].val.clusterDim.x, (unsigned)((npairs + G4_SLOTS - 1) / G4_SLOTS));
+  cfg.blockDim = dim3(G4_THREADS);
+  cfg.dynamicSmemBytes = sh;
+  cfg.stream = ctx->stream;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  // 16-byte loads need rows that start on 16 bytes
+  const int aligned = (reinterpret_cast<uintptr_t>(psi) & 15) == 0 && vol % 2 == 0;
+  return check_cuda(ctx, cudaLaunchKernelEx(&cfg, kern, reinterpret_cast<const float2*>(psi), N, vol, aligned, G),
+                    "gram4_kernel");
 }
 
 // One re-orthonormalisation of nconf configurations of N orbitals.
@@ -459,19 +645,16 @@ nrcps_status qr_reorthonormalise(nrcps_context* ctx, void* psi, int N, long vol,
       else if (N <= 32) launch(gram_tile_kernel<double, 3, true>);
       else if (db) launch(gram_tile_kernel<double, 9, true>);
       else launch(gram_tile_kernel<double, 9, false>);
-    } else if (N <= G4_ROWS) {
-      const size_t sh4 = sizeof(float2) * 2 * G4_ROWS * (GT + 1);
-      cudaFuncSetAttribute(gram4_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh4);
-      gram4_kernel<<<(unsigned)nconf, 256, sh4, ctx->stream>>>(psi, N, vol, G);
     } else {
-      if (N <= 22) launch(gram_tile_kernel<float, 2, true>);
-      else if (N <= 32) launch(gram_tile_kernel<float, 3, true>);
-      else launch(gram_tile_kernel<float, 9, true>);
+      NRCPS_TRY(launch_gram4(ctx, psi, N, vol, nconf, G));
     }
     ctx->launches++;
     NRCPS_TRY(check_launch(ctx, "gram_tile_kernel"));
   }
-  chol_inv_kernel<<<grid_for(nconf, 64), 64, 0, ctx->stream>>>(G, N, nconf, logR, prec == NRCPS_F32);
+  const size_t chol_sh = sizeof(double2) * N * N;
+  if (chol_sh > 48 * 1024)
+    cudaFuncSetAttribute(chol_inv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)chol_sh);
+  chol_inv_kernel<<<(unsigned)nconf, CHOL_THREADS, chol_sh, ctx->stream>>>(G, N, logR, prec == NRCPS_F32);
   ctx->launches++;
   NRCPS_TRY(check_launch(ctx, "chol_inv_kernel"));
   if (N <= 8) return launch_apply<8>(ctx, psi, N, vol, nconf, prec, G);
