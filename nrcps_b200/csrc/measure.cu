@@ -706,6 +706,225 @@ __global__ void __launch_bounds__(32 * kWarpLuMaxWarps) slater_dets_warp_kernel(
   }
 }
 
+// N <= 32: a segment of a warp per (matrix, measured minor) -- 8 lanes for
+// minors up to 8, 16 up to 16, the warp above -- lane i holding row i in
+// registers.  The elimination of slater_dets_warp_kernel; rows stay in their
+// lanes and carry their position instead of being swapped.  Column j is always
+// a[0]: a step's update writes entry k + 1 into place k, so the loop over j is
+// not unrolled and the code stays small (unrolled it would not fit the
+// instruction cache, with warps at different steps).  The pivot row and its
+// pivot's reciprocal (every row forms its own, beside the search) go through
+// shared memory.  Pivots are compared by |a|^2 / max|row|^2 -- the order of
+// |a| / max|row|, exact ties to the last position as before -- so that no
+// hypot is taken; where a square under- or overflows the moduli themselves are
+// compared.
+//
+// Bound by the latency of a step (search, reciprocal, broadcast) at 16 warps
+// per SM and by instruction issue (49 %): 4096 matrices of N = 19 take 186 us
+// (a warp per minor in shared memory: 507; a warp per minor in registers, no
+// segments: 319), 4096 of N = 7 with struck columns 30 (130), 500 of N = 32
+// 153 (345).
+constexpr int kRowLuWarps = 4;
+constexpr int kRowLuMax = 32;
+
+__device__ __forceinline__ double dnorm2(dc a) { return fma(a.re, a.re, a.im * a.im); }
+
+// The largest of v over the SEG lanes of a segment
+template <int SEG>
+__device__ __forceinline__ unsigned seg_max(unsigned v) {
+  if constexpr (SEG == 32) {
+    return __reduce_max_sync(0xffffffffu, v);
+  } else {
+#pragma unroll
+    for (int off = SEG / 2; off > 0; off >>= 1) v = max(v, __shfl_xor_sync(0xffffffffu, v, off));
+    return v;
+  }
+}
+
+// The minor of order n of configuration c (measured minor m), by the SEG lanes
+// of a segment; n = 0: none (a segment past the last minor).  Every segment of
+// a warp goes through the steps of the largest minor in it.  urow: the
+// segment's two pivot rows.
+template <int SEG, int NMAX, int MODE>
+__device__ __forceinline__ void minor_lu(const double2* __restrict__ S, const double2* __restrict__ psi1, int N,
+                                         long c, int m, int n, int log_det, double* __restrict__ out,
+                                         double2 (*urow)[NMAX + 1]) {
+  static_assert(NMAX % 4 == 0 && NMAX <= SEG, "rows live in lanes, columns in groups of four");
+  constexpr double kTiny = 1e-280, kHuge = 1e280;
+  const unsigned all = 0xffffffffu;
+  const int lane = threadIdx.x & (SEG - 1), first = (threadIdx.x & 31) & ~(SEG - 1);
+  const unsigned seg_mask = (SEG == 32 ? all : (1u << (SEG & 31)) - 1u) << first;
+  const int steps = SEG == 32 ? n : (int)__reduce_max_sync(all, (unsigned)n);
+  const int at = lane < n ? lane : 0;  // (lanes past the minor hold a copy of its first row, unused)
+  const double2* row = S + (c * N + at) * N;
+  dc a[NMAX];
+#pragma unroll
+  for (int k = 0; k < NMAX; ++k) a[k] = dc{0.0, 0.0};
+#pragma unroll
+  for (int k4 = 0; k4 < NMAX; k4 += 4) {
+    if (k4 >= steps) break;
+#pragma unroll
+    for (int k = k4; k < k4 + 4; ++k)
+      if (k < n) {
+        // SlaterDet2::Run column n - 1 from psi1[s + (n - 1) N] (slater_det2.C:102-106)
+        const double2* from = MODE && m % 2 == 0 && k == n - 1 ? psi1 + (c * N + n - 1) * N + at : row + k;
+        const double2 v = *from;
+        a[k] = dc{v.x, v.y};
+      }
+  }
+  double big = 0.0;  // the row's largest |a|^2
+#pragma unroll
+  for (int k = 0; k < NMAX; ++k) big = fmax(big, dnorm2(a[k]));
+  bool zero_row = lane < n && big == 0.0;
+  const bool plain = !(__ballot_sync(all, lane < n && !(big > kTiny && big < kHuge)) & seg_mask);
+  double inv_big = 1.0 / big;  // 1 / max|row|^2, or 1 / max|row| by moduli
+  if (!plain) {
+    big = 0.0;
+#pragma unroll
+    for (int k = 0; k < NMAX; ++k) big = fmax(big, dabs(a[k]));
+    zero_row = lane < n && big == 0.0;
+    inv_big = 1.0 / big;
+  }
+  const bool singular = __ballot_sync(all, zero_row) & seg_mask;
+  double d = 1.0;
+  dc mine{1.0, 0.0};  // the pivot of step `lane`
+  int pos = lane;     // this row's position after the swaps so far
+  for (int j = 0; j < steps; ++j) {
+    const int rem = steps - j;
+    const bool live = lane < n && pos >= j && j < n;
+    // the pivot this row would be, and its reciprocal
+    const bool zero = a[0].re == 0.0 && a[0].im == 0.0;
+    const dc z = zero ? dc{1.0e-20, 0.0} : a[0];
+    const double q = dnorm2(z);
+    double key = live && !zero ? (plain ? q : dabs(z)) * inv_big : 0.0;
+    unsigned hi = (unsigned)__double2hiint(key);
+    unsigned mhi = seg_max<SEG>(hi);
+    dc r;
+    {
+      const double inv = 1.0 / q;
+      r = dc{z.re * inv, -z.im * inv};
+      if (!(q > kTiny && q < kHuge)) r = drecip(z);
+    }
+    if (__any_sync(all, plain && j < n && mhi < 0x05000000u)) {
+      // every square of a segment below 1e-284 of its row's: compare its moduli
+      const bool low = plain && mhi < 0x05000000u;
+      if (low) key = live && !zero ? dabs(z) * sqrt(inv_big) : 0.0;
+      hi = (unsigned)__double2hiint(key);
+      mhi = seg_max<SEG>(hi);
+    }
+    unsigned cand = __ballot_sync(all, live && hi == mhi) & seg_mask;
+    if (__any_sync(all, cand & (cand - 1))) {  // more than one: the keys' lower halves, then the last position
+      const unsigned lo = (unsigned)__double2loint(key);
+      const bool in = live && hi == mhi;
+      const unsigned mlo = seg_max<SEG>(in ? lo : 0u);
+      const unsigned last = seg_max<SEG>(in && lo == mlo ? (unsigned)pos + 1u : 0u);
+      cand = __ballot_sync(all, in && lo == mlo && (unsigned)pos + 1u == last) & seg_mask;
+    }
+    const int at_lane = cand ? __ffs(cand) - 1 : first;
+    const bool pivot = live && (int)(threadIdx.x & 31) == at_lane;
+    double2* u = urow[j & 1];
+    if (pivot) {
+      u[NMAX] = make_double2(r.re, r.im);
+      u[0] = make_double2(z.re, z.im);
+#pragma unroll
+      for (int k4 = 0; k4 < NMAX; k4 += 4) {
+        if (k4 >= rem) break;
+#pragma unroll
+        for (int k = k4; k < k4 + 4; ++k)
+          if (k > 0) u[k] = make_double2(a[k].re, a[k].im);
+      }
+    }
+    const int imax = __shfl_sync(all, pos, at_lane);
+    if (imax != j) {
+      if (j < n) d = -d;
+      if (live && pos == j) pos = imax;  // (the pivot row takes position j)
+    }
+    if (pivot) pos = j;
+    __syncwarp();
+    if (lane == j && j < n) mine = dc{u[0].x, u[0].y};
+    const dc l = dmul(a[0], dc{u[NMAX].x, u[NMAX].y});  // (rows above are eliminated too, unread)
+#pragma unroll
+    for (int k4 = 0; k4 < NMAX; k4 += 4) {
+      if (k4 + 1 >= rem) break;
+#pragma unroll
+      for (int k = k4; k < k4 + 4; ++k) {
+        if (k + 1 < NMAX) {
+          const double2 w = u[k + 1];
+          a[k] = dc{fma(-l.re, w.x, fma(l.im, w.y, a[k + 1].re)), fma(-l.re, w.y, fma(-l.im, w.x, a[k + 1].im))};
+        }
+      }
+    }
+  }
+  // the product (or the sum of logs) of the pivots
+  dc v = mine;
+  if (log_det) v = lane < n ? dc{log(dabs(mine)), atan2(mine.im, mine.re)} : dc{0.0, 0.0};
+#pragma unroll
+  for (int off = SEG / 2; off > 0; off >>= 1) {
+    const dc w{__shfl_xor_sync(all, v.re, off), __shfl_xor_sync(all, v.im, off)};
+    v = log_det ? dc{v.re + w.re, v.im + w.im} : dmul(v, w);
+  }
+  if (lane == 0 && n > 0) {
+    if (singular) v = dc{nan(""), nan("")};  // an all-zero row: flagged to the host
+    else if (log_det) v.im += d < 0 ? 3.14159265358979323846 : 0.0;
+    else v = dc{d * v.re, d * v.im};
+    out[2L * m] = v.re;
+    out[2L * m + 1] = v.im;
+  }
+  __syncwarp();  // the pivot rows have been read
+}
+
+// Minors of orders lo + 1 .. hi of every configuration, SEG lanes each, by the
+// blocks b0, b0 + 1, .. of a launch
+template <int SEG, int NMAX, int MODE>
+__device__ __forceinline__ void minor_class(const double2* S, const double2* psi1, int N, int nconf, int lo, int hi,
+                                            int log_det, double* out, long out_conf_stride, long block,
+                                            double2* smem) {
+  constexpr int PER = 32 / SEG;
+  const int warp = threadIdx.x >> 5, seg = (threadIdx.x & 31) / SEG;
+  const int per_conf = (MODE ? 2 : 1) * (hi - lo);
+  const long g = (block * kRowLuWarps + warp) * PER + seg;
+  long c = g / per_conf;
+  int m = (MODE ? 2 * lo : lo) + (int)(g - c * per_conf);
+  int n = (MODE ? m / 2 : m) + 1;
+  if (c >= nconf) c = nconf - 1, n = 0;
+  minor_lu<SEG, NMAX, MODE>(S, psi1, N, c, m, n, log_det, out + c * out_conf_stride,
+                            reinterpret_cast<double2(*)[NMAX + 1]>(smem + (warp * PER + seg) * 2 * (NMAX + 1)));
+}
+
+__host__ __device__ inline long minor_blocks(int nconf, int mode, int lo, int hi, int per) {
+  const long segs = (long)nconf * (mode ? 2 : 1) * (hi > lo ? hi - lo : 0), w = (segs + per - 1) / per;
+  return (w + kRowLuWarps - 1) / kRowLuWarps;
+}
+
+// NMAX: N rounded up to a multiple of four; the first blocks take the largest minors
+template <int NMAX, int MODE>
+__global__ void __launch_bounds__(32 * kRowLuWarps, NMAX <= 8 ? 5 : NMAX <= 20 ? 4 : 2)
+    slater_dets_row_kernel(const double2* __restrict__ S, const double2* __restrict__ psi1, int N, int nconf,
+                           int log_det, double* __restrict__ out, long out_conf_stride) {
+  // one segment of 32 (NMAX + 1) or two of 16 or four of 8 (9) entries per warp, two rows each
+  __shared__ double2 smem[kRowLuWarps * 2 * (NMAX + 1 > 36 ? NMAX + 1 : 36)];
+  long b = blockIdx.x;
+  if constexpr (NMAX > 16) {
+    const long nb = minor_blocks(nconf, MODE, 16, N, 1);
+    if (b < nb) {
+      minor_class<32, NMAX, MODE>(S, psi1, N, nconf, 16, N, log_det, out, out_conf_stride, b, smem);
+      return;
+    }
+    b -= nb;
+  }
+  if constexpr (NMAX > 8) {
+    const int hi = N < 16 ? N : 16;
+    const long nb = minor_blocks(nconf, MODE, 8, hi, 2);
+    if (b < nb) {
+      minor_class<16, NMAX < 16 ? NMAX : 16, MODE>(S, psi1, N, nconf, 8, hi, log_det, out, out_conf_stride, b, smem);
+      return;
+    }
+    b -= nb;
+  }
+  minor_class<8, NMAX < 8 ? NMAX : 8, MODE>(S, psi1, N, nconf, 0, N < 8 ? N : 8, log_det, out, out_conf_stride, b,
+                                            smem);
+}
+
 constexpr int kWarpLuMaxN = 64;
 constexpr size_t kWarpLuSmemCap = 200 * 1024;
 
@@ -715,12 +934,32 @@ static int warp_lu_warps(int N) {
   return w < 1 ? 1 : (w > kWarpLuMaxWarps ? kWarpLuMaxWarps : w);
 }
 
-// Leading-minor determinants through the warp kernel (N <= 64, no scratch).
+// Leading-minor determinants by a warp per minor (N <= 64, no scratch): rows in
+// registers up to N = 32, the minor in shared memory above.
 nrcps_status slater_dets_warp(nrcps_context* ctx, const double* S, const double* psi1, int N, int nconf, int mode,
                               int log_det, double* out, long out_conf_stride, long out_offset) {
   const int nmeas = mode ? 2 * N : N;
   const long total = (long)nconf * nmeas;
   if (total == 0) return NRCPS_OK;
+  if (N <= kRowLuMax) {
+    const long blocks = minor_blocks(nconf, mode, 16, N, 1) + minor_blocks(nconf, mode, 8, N < 16 ? N : 16, 2) +
+                        minor_blocks(nconf, mode, 0, N < 8 ? N : 8, 4);
+    auto launch = [&](auto kern) {
+      kern<<<(unsigned)blocks, 32 * kRowLuWarps, 0, ctx->stream>>>(
+          reinterpret_cast<const double2*>(S), reinterpret_cast<const double2*>(psi1), N, nconf, log_det,
+          out + out_offset, out_conf_stride);
+    };
+#define NRCPS_CASE(M) \
+  if (N <= M) {       \
+    if (mode) launch(slater_dets_row_kernel<M, 1>); \
+    else launch(slater_dets_row_kernel<M, 0>);      \
+  }
+    NRCPS_CASE(4) else NRCPS_CASE(8) else NRCPS_CASE(12) else NRCPS_CASE(16) else NRCPS_CASE(20) else NRCPS_CASE(24)
+    else NRCPS_CASE(32)
+#undef NRCPS_CASE
+    ctx->launches++;
+    return check_launch(ctx, "slater_dets_row_kernel");
+  }
   static bool attr_set[16] = {false};
   if (!attr_set[ctx->device & 15]) {
     NRCPS_TRY(check_cuda(ctx,
