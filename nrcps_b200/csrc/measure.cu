@@ -9,64 +9,167 @@ namespace nrcps {
 namespace cg = cooperative_groups;
 
 // ---------------------------------------------------------------- overlap
-// One block per (configuration, orbital t); sources in chunks of 8.  FP64
-// accumulation for both orbital precisions.
+// S[c][s][t] = sum_p conj(src_s(p)) psi_{c,t}(p) in FP64 for both orbital
+// precisions.  A CTA takes a chunk of one configuration's sites and a tile of
+// up to 32 blocks of 4 sources x 4 orbitals; stages of T sites of all its
+// rows pass through shared memory (cp.async, two buffers), thread (block, l)
+// sums its block over the sites l, l + lanes, ..: 8 sixteen-byte loads for 64
+// FP64 FMAs.  Up to eight chunks are a cluster, which sums them; of more, each
+// chunk's sums go to `out` by themselves and overlap_sum_kernel adds them up.
+// Both in chunk order.
+//
+// Why chunks: one configuration's overlap is 47 M FP64 FMAs at N = 19, L = 32,
+// 3 us of the whole chip, and the reference's drivers measure one
+// configuration at a time.  Measured (FP64, call by call): that one 40 us, most
+// of it launch and latency (a block per orbital: 226); 64 configurations 0.54
+// ms against 1.64, 3.0 G FMAs at 30 % of the FP64 pipe, where the shared-memory
+// loads (45 %), the barriers of a stage and the FMAs take turns.
+constexpr int OV_THREADS = 256;
+
+struct OvTile {
+  int ts, tt;        // blocks of a tile along sources and orbitals
+  int ns_t, nt_t;    // tiles along each
+  int rows, T, lanes;
+  int log_t;         // T = 1 << log_t
+};
+__host__ __device__ inline OvTile overlap_tiles(int ns, int nt) {
+  OvTile o;
+  const int bs = (ns + 3) / 4, bt = (nt + 3) / 4;
+  if (bs * bt <= 32) {
+    o.ts = bs, o.tt = bt;
+  } else {  // near-equal tiles of at most 5 x 6 blocks
+    const int ks = (bs + 4) / 5, kt = (bt + 5) / 6;
+    o.ts = (bs + ks - 1) / ks, o.tt = (bt + kt - 1) / kt;
+  }
+  o.ns_t = (bs + o.ts - 1) / o.ts, o.nt_t = (bt + o.tt - 1) / o.tt;
+  o.rows = 4 * (o.ts + o.tt);
+  o.log_t = o.rows <= 8 ? 7 : o.rows <= 48 ? 6 : 5;  // both buffers of two CTAs fit an SM up to 48 rows
+  o.T = 1 << o.log_t;
+  o.lanes = 8;
+  while (2 * o.lanes * o.ts * o.tt <= OV_THREADS && 2 * o.lanes <= 32) o.lanes *= 2;
+  return o;
+}
+
 template <typename R>
-__global__ void __launch_bounds__(256) overlap_kernel(const double* __restrict__ src, int ns,
-                                                      const void* __restrict__ psi, int nt, long vol,
-                                                      double* __restrict__ S) {
-  const long ct = blockIdx.x;  // conf * nt + t
-  const long conf = ct / nt;
-  const int t = (int)(ct % nt);
-  const char* p = reinterpret_cast<const char*>(psi) + (size_t)ct * vol * 2 * sizeof(R);
-  __shared__ double red[8][2][8];
-  for (int s0 = 0; s0 < ns; s0 += 8) {
-    double ar[8], ai[8];
+__global__ void __launch_bounds__(OV_THREADS) overlap_tile_kernel(const double2* __restrict__ src, int ns,
+                                                                  const void* __restrict__ psi, int nt, long vol,
+                                                                  int chunks, long chunk_sites, OvTile o,
+                                                                  double2* __restrict__ out) {
+  extern __shared__ __align__(16) double2 ovs[];  // [2][rows][T]
+  const int T = o.T, lanes = o.lanes;
+  const long conf = blockIdx.x / chunks;
+  const int chunk = (int)(blockIdx.x - conf * chunks);
+  const int s0 = 4 * o.ts * (int)(blockIdx.y % o.ns_t), t0 = 4 * o.tt * (int)(blockIdx.y / o.ns_t);
+  const long p0 = chunk * chunk_sites, p1 = p0 + chunk_sites < vol ? p0 + chunk_sites : vol;
+  const cplx<R>* orb = reinterpret_cast<const cplx<R>*>(psi) + (size_t)conf * nt * vol;
+  const int l = threadIdx.x % lanes, slot = threadIdx.x / lanes;
+  const bool active = slot < o.ts * o.tt;
+  const int bi = active ? slot / o.tt : 0, bj = active ? slot % o.tt : 0;
+  auto fill = [&](long p, double2* t) {
+    for (int e = threadIdx.x; e < o.rows * T; e += OV_THREADS) {
+      const int r = e >> o.log_t;
+      const long q = p + (e & (T - 1));
+      const bool is_src = r < 4 * o.ts;
+      const int i = is_src ? s0 + r : t0 + r - 4 * o.ts;
+      if (q >= p1 || i >= (is_src ? ns : nt)) {
+        t[e] = make_double2(0.0, 0.0);
+      } else if (is_src || sizeof(R) == 8) {
+        const void* g = is_src ? (const void*)(src + (size_t)i * vol + q) : (const void*)(orb + (size_t)i * vol + q);
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(t + e)), "l"(g)
+                     : "memory");
+      } else {
+        const cplx<R> v = orb[(size_t)i * vol + q];
+        t[e] = make_double2((double)v.re, (double)v.im);
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  double re[16], im[16];
 #pragma unroll
-    for (int k = 0; k < 8; ++k) ar[k] = ai[k] = 0.0;
-    for (long i = threadIdx.x; i < vol; i += blockDim.x) {
-      cplx<R> q = ld<R>(p, i);
-      double qr = (double)q.re, qi = (double)q.im;
+  for (int k = 0; k < 16; ++k) re[k] = im[k] = 0.0;
+  const int size = o.rows * T;
+  fill(p0, ovs);
+  int buf = 0;
+  for (long p = p0; p < p1; p += T, buf ^= 1) {
+    __syncthreads();  // every thread is done with the buffer the next copies overwrite
+    if (p + T < p1) fill(p + T, ovs + (buf ^ 1) * size);
+    else asm volatile("cp.async.commit_group;" ::: "memory");
+    asm volatile("cp.async.wait_group 1;" ::: "memory");
+    __syncthreads();
+    if (active) {
+      const double2* ta = ovs + buf * size + 4 * bi * T;
+      const double2* tb = ovs + buf * size + 4 * (o.ts + bj) * T;
+      for (int q = l; q < T; q += lanes) {
+        double2 b[4];
 #pragma unroll
-      for (int k = 0; k < 8; ++k) {
-        if (s0 + k < ns) {
-          double2 a = reinterpret_cast<const double2*>(src)[(long)(s0 + k) * vol + i];
-          ar[k] = fma(a.x, qr, ar[k]);  // two fused multiply-adds per component
-          ar[k] = fma(a.y, qi, ar[k]);
-          ai[k] = fma(a.x, qi, ai[k]);
-          ai[k] = fma(-a.y, qr, ai[k]);
+        for (int v = 0; v < 4; ++v) b[v] = tb[v * T + q];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const double2 a = ta[u * T + q];
+#pragma unroll
+          for (int v = 0; v < 4; ++v) {
+            re[4 * u + v] = fma(a.x, b[v].x, re[4 * u + v]);
+            im[4 * u + v] = fma(a.x, b[v].y, im[4 * u + v]);
+          }
+#pragma unroll
+          for (int v = 0; v < 4; ++v) {
+            re[4 * u + v] = fma(a.y, b[v].y, re[4 * u + v]);
+            im[4 * u + v] = fma(-a.y, b[v].x, im[4 * u + v]);
+          }
         }
       }
     }
-    // warp reduce then block reduce
+  }
+  // the lanes of a block are neighbours in one warp
+  for (int off = lanes / 2; off > 0; off >>= 1)
 #pragma unroll
-    for (int k = 0; k < 8; ++k) {
-      for (int off = 16; off > 0; off >>= 1) {
-        ar[k] += __shfl_down_sync(0xffffffffu, ar[k], off);
-        ai[k] += __shfl_down_sync(0xffffffffu, ai[k], off);
-      }
+    for (int k = 0; k < 16; ++k) {
+      re[k] += __shfl_xor_sync(0xffffffffu, re[k], off);
+      im[k] += __shfl_xor_sync(0xffffffffu, im[k], off);
     }
-    const int warp = threadIdx.x >> 5, ln = threadIdx.x & 31;
-    if (ln == 0) {
+  cg::cluster_group cluster = cg::this_cluster();
+  const int split = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
+  if (split == 1) {
+    if (active && l == 0)
 #pragma unroll
-      for (int k = 0; k < 8; ++k) {
-        red[warp][0][k] = ar[k];
-        red[warp][1][k] = ai[k];
+      for (int k = 0; k < 16; ++k) {
+        const int s = s0 + 4 * bi + k / 4, t = t0 + 4 * bj + k % 4;
+        if (s < ns && t < nt) out[((size_t)blockIdx.x * ns + s) * nt + t] = make_double2(re[k], im[k]);
       }
+    return;
+  }
+  // a cluster holds all chunks of its configuration: entries spread over its CTAs
+  __syncthreads();
+  if (active && l == 0)
+#pragma unroll
+    for (int k = 0; k < 16; ++k) ovs[16 * slot + k] = make_double2(re[k], im[k]);
+  cluster.sync();
+  for (int e = rank * OV_THREADS + threadIdx.x; e < 16 * o.ts * o.tt; e += split * OV_THREADS) {
+    double2 v = make_double2(0.0, 0.0);
+    for (int r = 0; r < split; ++r) {
+      const double2 w = cluster.map_shared_rank(ovs, r)[e];
+      v.x += w.x;
+      v.y += w.y;
     }
-    __syncthreads();
-    if (threadIdx.x < 8 && s0 + (int)threadIdx.x < ns) {
-      const int k = threadIdx.x;
-      double sr = 0.0, si = 0.0;
-      for (int w = 0; w < (int)(blockDim.x >> 5); ++w) {
-        sr += red[w][0][k];
-        si += red[w][1][k];
-      }
-      long o = ((conf * ns + (s0 + k)) * (long)nt + t) * 2;
-      S[o] = sr;
-      S[o + 1] = si;
+    const int b = e / 16, s = s0 + 4 * (b / o.tt) + e % 16 / 4, t = t0 + 4 * (b % o.tt) + e % 4;
+    if (s < ns && t < nt) out[((size_t)conf * ns + s) * nt + t] = v;
+  }
+  cluster.sync();  // peers keep their shared memory until every sum is read
+}
+
+// S[c][e] = sum over the chunks, in order
+__global__ void overlap_sum_kernel(const double2* __restrict__ part, int chunks, long per_conf, long total,
+                                   double2* __restrict__ S) {
+  for (long e = (long)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (long)gridDim.x * blockDim.x) {
+    const long c = e / per_conf, i = e - c * per_conf;
+    const double2* p = part + (size_t)c * chunks * per_conf + i;
+    double2 v = make_double2(0.0, 0.0);
+    for (int k = 0; k < chunks; ++k) {
+      const double2 w = p[(size_t)k * per_conf];
+      v.x += w.x;
+      v.y += w.y;
     }
-    __syncthreads();
+    S[e] = v;
   }
 }
 
@@ -1009,14 +1112,71 @@ nrcps_status slater_dets_dispatch(nrcps_context* ctx, const double* S, const dou
   return slater_dets_impl(ctx, S, psi1, N, nconf, mode, log_det, out, out_conf_stride, out_offset, scr);
 }
 
+// The chunks' sums of overlap_tile_kernel: a buffer of fixed size, made at the
+// first use outside a stream capture.
+constexpr size_t kOverlapPartBytes = 16u << 20;
+nrcps_status overlap_reserve(nrcps_context* ctx) {
+  if (ctx->overlap_part) return NRCPS_OK;
+  return check_cuda(ctx, cudaMalloc(&ctx->overlap_part, kOverlapPartBytes), "cudaMalloc(overlap sums)");
+}
+
+template <typename R>
+static nrcps_status launch_overlap(nrcps_context* ctx, const double* src, int ns, const void* psi, int nt, int nconf,
+                                   long vol, double* S) {
+  const OvTile o = overlap_tiles(ns, nt);
+  const size_t smem = sizeof(double2) * 2 * (size_t)o.rows * o.T;
+  NRCPS_TRY(check_cuda(ctx, cudaFuncSetAttribute(overlap_tile_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                 (int)smem),
+                       "overlap_tile: smem attribute"));
+  // chunks: about four CTAs per SM, at least eight stages each, and what the buffer holds
+  const int tiles = o.ns_t * o.nt_t;
+  const size_t per_chunk = sizeof(double2) * (size_t)nconf * ns * nt;
+  long chunks = (4L * ctx->sm_count + (long)nconf * tiles - 1) / ((long)nconf * tiles);
+  if (chunks > vol / (8L * o.T)) chunks = vol / (8L * o.T);
+  if (chunks > (long)(kOverlapPartBytes / per_chunk)) chunks = (long)(kOverlapPartBytes / per_chunk);
+  if (chunks > 8 && chunks <= 16) chunks = 8;  // (the second kernel costs more than it gives)
+  if (chunks > 8 && !ctx->overlap_part) {
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    cudaStreamIsCapturing(ctx->stream, &cs);
+    if (cs != cudaStreamCaptureStatusNone) chunks = 8;  // nothing is allocated inside a capture
+    else NRCPS_TRY(overlap_reserve(ctx));
+  }
+  if (chunks < 1) chunks = 1;
+  const long sites = (vol + chunks - 1) / chunks;
+  const long chunk_sites = (sites + o.T - 1) / o.T * o.T;
+  chunks = (vol + chunk_sites - 1) / chunk_sites;
+  const bool sums = chunks > 8;
+  double2* out = reinterpret_cast<double2*>(sums ? (double*)ctx->overlap_part : S);
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = sums ? 1u : (unsigned)chunks;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cfg.gridDim = dim3((unsigned)(nconf * chunks), (unsigned)tiles);
+  cfg.blockDim = dim3(OV_THREADS);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = ctx->stream;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  ctx->launches++;
+  NRCPS_TRY(check_cuda(ctx, cudaLaunchKernelEx(&cfg, overlap_tile_kernel<R>, reinterpret_cast<const double2*>(src), ns,
+                                               psi, nt, vol, (int)chunks, chunk_sites, o, out),
+                       "overlap_tile_kernel launch"));
+  if (sums) {
+    const long per_conf = (long)ns * nt, total = nconf * per_conf;
+    overlap_sum_kernel<<<grid_for(total, 64), 64, 0, ctx->stream>>>(out, (int)chunks, per_conf, total,
+                                                                    reinterpret_cast<double2*>(S));
+    ctx->launches++;
+    NRCPS_TRY(check_launch(ctx, "overlap_sum_kernel"));
+  }
+  return NRCPS_OK;
+}
+
 nrcps_status overlap_impl(nrcps_context* ctx, const double* src, int ns, const void* psi, int nt, int nconf,
                           long vol, nrcps_precision prec, double* S) {
-  long blocks = (long)nconf * nt;
-  if (blocks == 0) return NRCPS_OK;
-  if (prec == NRCPS_F64) overlap_kernel<double><<<(unsigned)blocks, 256, 0, ctx->stream>>>(src, ns, psi, nt, vol, S);
-  else overlap_kernel<float><<<(unsigned)blocks, 256, 0, ctx->stream>>>(src, ns, psi, nt, vol, S);
-  ctx->launches++;
-  return check_launch(ctx, "overlap_kernel");
+  if ((long)nconf * nt * ns == 0) return NRCPS_OK;
+  return prec == NRCPS_F64 ? launch_overlap<double>(ctx, src, ns, psi, nt, nconf, vol, S)
+                           : launch_overlap<float>(ctx, src, ns, psi, nt, nconf, vol, S);
 }
 
 nrcps_status gather_impl(nrcps_context* ctx, const int* index, int ns, const void* psi, int nt, int nconf, long vol,
