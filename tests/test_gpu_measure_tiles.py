@@ -65,9 +65,9 @@ def test_minors_by_segments_against_the_thread_kernel(ctx, N, mode, log):
         assert np.max(np.abs(a.real - b.real)) < 1e-9
         assert np.max(np.abs(np.exp(1j * a.imag) - np.exp(1j * b.imag))) < 1e-9
         return
-    ok = np.isfinite(a) & np.isfinite(b) & (np.abs(b) > 1e-290)
+    ok = np.isfinite(b) & (np.abs(b) > 1e-290)
     assert ok[np.arange(37) != 5][:5].all()
-    assert np.max(np.abs(a - b)[ok] / np.abs(b)[ok]) < 1e-11
+    assert np.max(np.abs(a[ok] - b[ok]) / np.abs(b[ok])) < 1e-11
 
 
 def test_minors_ties_zero_pivots_and_zero_rows(ctx):
