@@ -365,7 +365,7 @@ class Propagator:
 
     def set(self, psi, n: int) -> None:
         src = psi if isinstance(psi, torch.Tensor) else torch.from_numpy(np.asarray(psi))
-        self.b.get(n).copy_(src.reshape(self.b.dims).to(self.b.b.dtype).to(self.ctx.device))
+        self.b.get(n).copy_(src.reshape(self.b.dims))  # (converts on the way)
 
     def get(self, n: Optional[int] = None):
         return self.b if n is None else self.b.get(n)

@@ -91,6 +91,8 @@ extern "C" nrcps_status nrcps_destroy(nrcps_context* ctx) {
   if (ctx->kin_f32) cudaFree(ctx->kin_f32);
   if (ctx->zpos) cudaFree(ctx->zpos);
   if (ctx->tc_split) cudaFree(ctx->tc_split);
+  for (void* u : ctx->unit)
+    if (u) cudaFree(u);
   if (ctx->overlap_part) cudaFree(ctx->overlap_part);
   if (ctx->dev_err) cudaFree(ctx->dev_err);
   delete ctx;

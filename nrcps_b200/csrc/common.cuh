@@ -112,6 +112,7 @@ struct Context {
   // TF32 hi / lo split of the sources for nrcps_overlap's tensor-core path (grown on demand)
   void* tc_split = nullptr;
   size_t tc_split_bytes = 0;
+  void* unit[64] = {};  // tables of ones for a fused step without k(p) or field, by lattice extent
   void* overlap_part = nullptr;  // chunk sums of the CUDA-core overlap (fixed size, made at the first use)
   int* dev_err = nullptr;
   int* dev_pair_flag = nullptr;  // the word after dev_err: 1 = the last checked opposite-site table is no involution  // device flag set by kernels whose bounded waits time out

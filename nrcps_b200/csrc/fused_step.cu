@@ -1380,8 +1380,8 @@ struct FusedVariant {
 static const FusedVariant kVariants[] = {
     {NRCPS_F32, 8, 1, 4, launch_fused<float, 8, 1, 4>},
     {NRCPS_F32, 8, 1, 0, launch_fused<float, 8, 1>},
-    {NRCPS_F32, 16, 1, 4, launch_fused<float, 16, 1, 4>},
     {NRCPS_F32, 16, 1, 0, launch_fused<float, 16, 1>},
+    {NRCPS_F32, 16, 1, 4, launch_fused<float, 16, 1, 4>},
     {NRCPS_F32, 16, 2, 2, launch_fused<float, 16, 2, 2>},
     {NRCPS_F32, 16, 2, 9, launch_fused<float, 16, 2, 9>},
     {NRCPS_F32, 16, 2, 10, launch_fused<float, 16, 2, 10>},
@@ -1422,15 +1422,15 @@ static const FusedVariant kVariants[] = {
     {NRCPS_F32, 48, 16, 3, launch_fused<float, 48, 16, 3>},
     {NRCPS_F32, 48, 16, 1, launch_fused<float, 48, 16, 1>},
     {NRCPS_F64, 8, 1, 0, launch_fused<double, 8, 1>},
-    {NRCPS_F64, 16, 2, 2, launch_fused<double, 16, 2, 2>},
     {NRCPS_F64, 16, 2, 0, launch_fused<double, 16, 2>},
+    {NRCPS_F64, 16, 2, 2, launch_fused<double, 16, 2, 2>},
     {NRCPS_F64, 16, 2, 1, launch_fused<double, 16, 2, 1>},
+    {NRCPS_F64, 24, 4, 11, launch_fused<double, 24, 4, 11>},
     {NRCPS_F64, 24, 4, 2, launch_fused<double, 24, 4, 2>},
     {NRCPS_F64, 24, 4, 0, launch_fused<double, 24, 4>},
-    {NRCPS_F64, 24, 4, 11, launch_fused<double, 24, 4, 11>},
+    {NRCPS_F64, 32, 16, 11, launch_fused<double, 32, 16, 11>},
     {NRCPS_F64, 32, 16, 3, launch_fused<double, 32, 16, 3>},
     {NRCPS_F64, 32, 16, 7, launch_fused<double, 32, 16, 7>},
-    {NRCPS_F64, 32, 16, 11, launch_fused<double, 32, 16, 11>},
     {NRCPS_F64, 32, 16, 0, launch_fused<double, 32, 16>},
     {NRCPS_F64, 32, 8, 0, launch_fused<double, 32, 8>},
     {NRCPS_F64, 32, 16, 2, launch_fused<double, 32, 16, 2>},

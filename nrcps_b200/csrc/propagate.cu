@@ -26,7 +26,7 @@ struct PencilGeom {
 enum PencilOp { OP_NONE = 0, OP_PRE_MUL = 1, OP_POST_MUL = 2, OP_MID_FIELD = 3 };
 
 struct FieldArgs {
-  int mode;              // 0 complex fld, 1 Z2 bits, 2 interleaved complex phi, 3 real FP32 weights
+  int mode;              // 0 complex fld, 1 Z2 bits, 2 interleaved complex phi, 3 real FP32 weights, 4 none (pos alone)
   const void* field;
   uint64_t bit0;         // element (mode 0/2) or bit (mode 1) offset of configuration 0
   uint64_t conf_stride;  // elements or bits between configurations
@@ -40,6 +40,7 @@ struct FieldArgs {
 template <typename R>
 __device__ __forceinline__ cplx<R> field_factor(const FieldArgs& f, long conf, long site) {
   cplx<R> w;
+  if (f.mode == 4) return cplx<R>{(R)f.pos[site], (R)0};
   const uint64_t k = f.bit0 + (f.conf_base ? f.conf_base[conf] : (uint64_t)conf * f.conf_stride) + (uint64_t)site;
   if (f.mode == 0) {
     double2 v = reinterpret_cast<const double2*>(f.field)[k];
@@ -192,24 +193,10 @@ __global__ void div_real_kernel(void* psi, long n, long vol, const double* xi) {
   }
 }
 
-template <typename R>
-__global__ void mul_real_kernel(void* psi, long n, long vol, const double* v) {
+__global__ void mul_real_kernel(double* fld, long n, const double* v) {
   for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
-    cplx<R> a = ld<R>(psi, i);
-    R k = (R)v[i % vol];
-    a.re *= k;
-    a.im *= k;
-    st<R>(psi, i, a);
-  }
-}
-
-template <typename R>
-__global__ void mul_complex_kernel(void* psi, long n, long vol, const double* fld) {
-  for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
-    cplx<R> a = ld<R>(psi, i);
-    double2 f = reinterpret_cast<const double2*>(fld)[i % vol];
-    cplx<R> w{(R)f.x, (R)f.y};
-    st<R>(psi, i, cmul(w, a));
+    fld[2 * i] *= v[i];
+    fld[2 * i + 1] *= v[i];
   }
 }
 
@@ -252,20 +239,114 @@ extern "C" nrcps_status nrcps_kinetic_evolve(nrcps_context* ctx, void* psi, int 
   return check_launch(ctx, "div_real_kernel");
 }
 
+namespace nrcps {
+bool fused_supported(nrcps_precision prec, const int d[3]);
+nrcps_status fused_step(nrcps_context* ctx, void* psi, int batch, int nconf, const int d[3], const void* kin_table,
+                        nrcps_precision prec, const nrcps_position_factor* w, int cluster, const void* zpos);
+bool evolve_fits(nrcps_precision prec, const int d[3]);  // evolve.cu
+nrcps_status evolve_step(nrcps_context* ctx, void* psi, int batch, const int d[3], const double* w, bool w_complex,
+                         nrcps_precision prec);
+nrcps_status evolve_initialize(nrcps_context* ctx, const double* phi, const double* c, const int d[3], double* fld);
+
+// Tables of ones for the fused step: a field of V complex ones, k(p) as V
+// doubles, and as V (1, 0) float pairs
+__global__ void unit_table_kernel(double* t, long n) {
+  for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
+    reinterpret_cast<double2*>(t)[i] = make_double2(1.0, 0.0);
+    t[2 * n + i] = 1.0;
+    reinterpret_cast<float2*>(t + 3 * n)[i] = make_float2(1.f, 0.f);
+  }
+}
+
+// The tables for a cube of L^3 sites, one per context and lattice size, made at
+// their first use and kept (a captured graph may hold its address); NULL where it
+// would have to be made inside a stream capture.
+static const double* unit_table(nrcps_context* ctx, int L) {
+  void*& t = ctx->unit[L & 63];
+  if (t) return (const double*)t;
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  cudaStreamIsCapturing(ctx->stream, &cs);
+  if (cs != cudaStreamCaptureStatusNone) return nullptr;
+  const long V = (long)L * L * L;
+  void* p = nullptr;
+  if (cudaMalloc(&p, 32 * (size_t)V) != cudaSuccess) {
+    cudaGetLastError();
+    return nullptr;
+  }
+  unit_table_kernel<<<grid_for(V, 256), 256, 0, ctx->stream>>>((double*)p, V);
+  ctx->launches++;
+  // later calls may come on another stream
+  if (cudaStreamSynchronize(ctx->stream) != cudaSuccess) {
+    cudaFree(p);
+    return nullptr;
+  }
+  t = p;
+  return (const double*)t;
+}
+
+// The fused step with k(p) = 1 on a cubic lattice that has one: psi <-
+// B[w . F[psi]]; NRCPS_ERR_UNSUPPORTED where it does not serve.
+static nrcps_status evolve_fused(nrcps_context* ctx, void* psi, int batch, const int d[3], const double* w,
+                                 bool w_complex, nrcps_precision prec) {
+  if (!ctx->fused_enabled || !fused_supported(prec, d)) return NRCPS_ERR_UNSUPPORTED;
+  const long V = vol_of(d);
+  const double* unit = unit_table(ctx, d[0]);
+  if (!unit) return NRCPS_ERR_UNSUPPORTED;
+  nrcps_position_factor pf{};
+  pf.field_mode = 0;  // the factor fld(x) P(x)
+  pf.dev_field = w_complex ? w : unit;
+  pf.dev_pos = w_complex ? nullptr : w;
+  return fused_step(ctx, psi, batch, 1, d, unit + (prec == NRCPS_F64 ? 2 : 3) * V, prec, &pf, ctx->fused_cluster,
+                    nullptr);
+}
+
+// psi <- B[w . F[psi]], w complex (interleaved) or real FP64: one launch where
+// the fused step or a CTA's shared memory holds an orbital, else five pencil
+// passes.  At class-API sizes the launches are the time, per call: 19 FP64
+// orbitals at L = 32 25 us (seven launches: 56), 7 FP32 orbitals of 24 x 12 x 16
+// 14 (37), 2 of 8^3 12 (38), 10 FP32 orbitals at L = 48 45 (72).
+static nrcps_status evolve_any(nrcps_context* ctx, void* psi, int batch, const int d[3], const double* w,
+                               bool w_complex, nrcps_precision prec) {
+  const nrcps_status st = evolve_fused(ctx, psi, batch, d, w, w_complex, prec);
+  if (st != NRCPS_ERR_UNSUPPORTED) return st;
+  // (a CTA per orbital: past some waves of them the pencil passes' better
+  // occupancy wins, 2000 orbitals of 12^3 98 / 90 us)
+  if (evolve_fits(prec, d) && batch <= 6 * ctx->sm_count) return evolve_step(ctx, psi, batch, d, w, w_complex, prec);
+  FieldArgs none{}, f{};
+  f.mode = w_complex ? 0 : 4;
+  f.field = w;
+  f.pos = w_complex ? nullptr : w;
+  f.vol = (double)vol_of(d);
+  f.orbs_per_conf = batch;
+  auto passes = [&](auto zero) {
+    using R = decltype(zero);
+    NRCPS_TRY((launch_axis<R, -1, OP_NONE>(ctx, psi, batch, d, 2, nullptr, none)));
+    NRCPS_TRY((launch_axis<R, -1, OP_NONE>(ctx, psi, batch, d, 1, nullptr, none)));
+    NRCPS_TRY((launch_axis<R, -1, OP_MID_FIELD>(ctx, psi, batch, d, 0, nullptr, f)));
+    NRCPS_TRY((launch_axis<R, +1, OP_NONE>(ctx, psi, batch, d, 1, nullptr, none)));
+    return launch_axis<R, +1, OP_NONE>(ctx, psi, batch, d, 2, nullptr, none);
+  };
+  return prec == NRCPS_F64 ? passes(0.0) : passes(0.f);
+}
+
+// conj(lat), and conj of the result with the (1 + .) / V of Initialize
+__global__ void conj_kernel(double2* dst, const double2* src, long n) {
+  for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x)
+    dst[i] = make_double2(src[i].x, -src[i].y);
+}
+__global__ void conj_plus_one_div_vol_kernel(double2* fld, long vol) {
+  for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < vol; i += (long)gridDim.x * blockDim.x)
+    fld[i] = make_double2((fld[i].x + 1.0) / vol, -fld[i].y / vol);
+}
+}  // namespace nrcps
+
 extern "C" nrcps_status nrcps_potential_evolve(nrcps_context* ctx, void* psi, int batch, const int dims[3],
                                                const double* dev_pot, nrcps_precision prec) {
   if (!ctx) return NRCPS_ERR_INVALID_ARGUMENT;
   NRCPS_REQUIRE(ctx, (psi || batch == 0) && dev_pot && dims && batch >= 0, "nrcps_potential_evolve: bad arguments");
   NRCPS_TRY(check_dims(ctx, dims));
-  long vol = vol_of(dims), n = vol * batch;
-  if (n == 0) return NRCPS_OK;
-  NRCPS_TRY(fft3d_any(ctx, psi, batch, dims, prec, -1));
-  unsigned grid = grid_for(n, 256, (long)ctx->sm_count * 8);
-  if (prec == NRCPS_F64) mul_real_kernel<double><<<grid, 256, 0, ctx->stream>>>(psi, n, vol, dev_pot);
-  else mul_real_kernel<float><<<grid, 256, 0, ctx->stream>>>(psi, n, vol, dev_pot);
-  ctx->launches++;
-  NRCPS_TRY(check_launch(ctx, "mul_real_kernel"));
-  return fft3d_any(ctx, psi, batch, dims, prec, +1);
+  if (batch == 0) return NRCPS_OK;
+  return evolve_any(ctx, psi, batch, dims, dev_pot, false, prec);
 }
 
 extern "C" nrcps_status nrcps_interaction_evolve(nrcps_context* ctx, void* psi, int batch, const int dims[3],
@@ -273,15 +354,8 @@ extern "C" nrcps_status nrcps_interaction_evolve(nrcps_context* ctx, void* psi, 
   if (!ctx) return NRCPS_ERR_INVALID_ARGUMENT;
   NRCPS_REQUIRE(ctx, (psi || batch == 0) && dev_fld && dims && batch >= 0, "nrcps_interaction_evolve: bad arguments");
   NRCPS_TRY(check_dims(ctx, dims));
-  long vol = vol_of(dims), n = vol * batch;
-  if (n == 0) return NRCPS_OK;
-  NRCPS_TRY(fft3d_any(ctx, psi, batch, dims, prec, -1));
-  unsigned grid = grid_for(n, 256, (long)ctx->sm_count * 8);
-  if (prec == NRCPS_F64) mul_complex_kernel<double><<<grid, 256, 0, ctx->stream>>>(psi, n, vol, dev_fld);
-  else mul_complex_kernel<float><<<grid, 256, 0, ctx->stream>>>(psi, n, vol, dev_fld);
-  ctx->launches++;
-  NRCPS_TRY(check_launch(ctx, "mul_complex_kernel"));
-  return fft3d_any(ctx, psi, batch, dims, prec, +1);
+  if (batch == 0) return NRCPS_OK;
+  return evolve_any(ctx, psi, batch, dims, dev_fld, true, prec);
 }
 
 extern "C" nrcps_status nrcps_interaction_initialize(nrcps_context* ctx, const double* dev_lat,
@@ -290,26 +364,49 @@ extern "C" nrcps_status nrcps_interaction_initialize(nrcps_context* ctx, const d
   if (!ctx) return NRCPS_ERR_INVALID_ARGUMENT;
   NRCPS_REQUIRE(ctx, dev_lat && dev_itab && dev_fld && dims, "nrcps_interaction_initialize: bad arguments");
   NRCPS_TRY(check_dims(ctx, dims));
-  long vol = vol_of(dims);
+  const long vol = vol_of(dims);
+  // one field: a CTA does it up to 8192 sites, a cluster does a larger cube
+  // (as conj(B[c F[conj(phi)]]), c being real), pencil passes the rest
+  if (vol <= 8192 && evolve_fits(NRCPS_F64, dims)) return evolve_initialize(ctx, dev_lat, dev_itab, dims, dev_fld);
+  if (ctx->fused_enabled && fused_supported(NRCPS_F64, dims) && unit_table(ctx, dims[0]) &&
+      (reinterpret_cast<uintptr_t>(dev_fld) & 15) == 0 && (reinterpret_cast<uintptr_t>(dev_lat) & 15) == 0) {
+    conj_kernel<<<grid_for(vol, 256), 256, 0, ctx->stream>>>(reinterpret_cast<double2*>(dev_fld),
+                                                             reinterpret_cast<const double2*>(dev_lat), vol);
+    ctx->launches++;
+    NRCPS_TRY(check_launch(ctx, "conj_kernel"));
+    NRCPS_TRY(evolve_fused(ctx, dev_fld, 1, dims, dev_itab, false, NRCPS_F64));
+    conj_plus_one_div_vol_kernel<<<grid_for(vol, 256), 256, 0, ctx->stream>>>(reinterpret_cast<double2*>(dev_fld), vol);
+    ctx->launches++;
+    return check_launch(ctx, "conj_plus_one_div_vol_kernel");
+  }
   unsigned grid = grid_for(2 * vol, 256, (long)ctx->sm_count * 8);
   copy_kernel<<<grid, 256, 0, ctx->stream>>>(dev_fld, dev_lat, 2 * vol);
   ctx->launches++;
   NRCPS_TRY(check_launch(ctx, "copy_kernel"));
-  NRCPS_TRY(fft3d_t<double>(ctx, dev_fld, 1, dims, +1));
-  mul_real_kernel<double><<<grid_for(vol, 256), 256, 0, ctx->stream>>>(dev_fld, vol, vol, dev_itab);
-  ctx->launches++;
-  NRCPS_TRY(check_launch(ctx, "mul_real_kernel"));
-  NRCPS_TRY(fft3d_t<double>(ctx, dev_fld, 1, dims, -1));
+  FieldArgs none{}, f{};
+  f.mode = 4;
+  f.pos = dev_itab;
+  f.vol = (double)vol;
+  f.orbs_per_conf = 1;
+  NRCPS_TRY((launch_axis<double, +1, OP_NONE>(ctx, dev_fld, 1, dims, 2, nullptr, none)));
+  NRCPS_TRY((launch_axis<double, +1, OP_NONE>(ctx, dev_fld, 1, dims, 1, nullptr, none)));
+  if (dims[0] < 48) {
+    NRCPS_TRY((launch_axis<double, +1, OP_MID_FIELD>(ctx, dev_fld, 1, dims, 0, nullptr, f)));
+  } else {  // (two FP64 transforms of 48 in one thread spill; few pencils hide it badly: 70 us against 66)
+    NRCPS_TRY((launch_axis<double, +1, OP_NONE>(ctx, dev_fld, 1, dims, 0, nullptr, none)));
+    mul_real_kernel<<<grid_for(vol, 256), 256, 0, ctx->stream>>>(dev_fld, vol, dev_itab);
+    ctx->launches++;
+    NRCPS_TRY(check_launch(ctx, "mul_real_kernel"));
+    NRCPS_TRY((launch_axis<double, -1, OP_NONE>(ctx, dev_fld, 1, dims, 0, nullptr, none)));
+  }
+  NRCPS_TRY((launch_axis<double, -1, OP_NONE>(ctx, dev_fld, 1, dims, 1, nullptr, none)));
+  NRCPS_TRY((launch_axis<double, -1, OP_NONE>(ctx, dev_fld, 1, dims, 2, nullptr, none)));
   plus_one_div_vol_kernel<<<grid_for(vol, 256), 256, 0, ctx->stream>>>(dev_fld, vol);
   ctx->launches++;
   return check_launch(ctx, "plus_one_div_vol_kernel");
 }
 
 namespace nrcps {
-bool fused_supported(nrcps_precision prec, const int d[3]);
-nrcps_status fused_step(nrcps_context* ctx, void* psi, int batch, int nconf, const int d[3], const void* kin_table,
-                        nrcps_precision prec, const nrcps_position_factor* w, int cluster, const void* zpos);
-
 // The per-site weights of a Z2 field times a position factor P:
 // (1 + a) P/V and (1 - a) P/V, each split (hi, lo) into floats (float4 per
 // site) for FP32 orbitals, plain doubles (double2 per site) for FP64.
