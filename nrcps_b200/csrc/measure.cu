@@ -252,7 +252,8 @@ __global__ void __launch_bounds__(256) pair_kernel(const void* __restrict__ psi1
 // With psi1 = psi2 and a weight even under the pairing (w(opp(i)) = w(i),
 // TwoBody's tables), the pair of terms of i and opp(i) is symmetric in
 // (s, t), so phi is: only the blocks on and above the diagonal are summed
-// and each is written to both triangles.
+// and each is written to both triangles (FP32 orbitals with n = 9 .. 20 mostly
+// take pair_sym.cu instead).
 constexpr int PAIR_THREADS = 256;
 constexpr int PAIR_MAXN = 32;
 constexpr int PB = 2;                // register block: PB x PB complex pair-matrix entries per thread
@@ -340,7 +341,8 @@ template <typename R>
 __global__ void __launch_bounds__(PAIR_THREADS, 4)
     pair_tile_kernel(const void* __restrict__ psi1, const void* __restrict__ psi2, int n, long vol,
                      const double* __restrict__ w, const int* __restrict__ opp, const int* __restrict__ flags,
-                     int host_flags, int ts, double* __restrict__ phi) {
+                     int host_flags, int leave_sym, int ts, double* __restrict__ phi) {
+  if (leave_sym && !*flags) return;  // pair_sym_kernel's
   extern __shared__ __align__(16) unsigned char pair_smem[];
   const int LD = 2 * ts + 1;
   const int nb = (n + PB - 1) / PB, rows = nb * PB;
@@ -1193,7 +1195,7 @@ nrcps_status gather_impl(nrcps_context* ctx, const int* index, int ns, const voi
 template <typename R>
 static nrcps_status launch_pair_tile(nrcps_context* ctx, const void* psi1, const void* psi2, int n, int nconf,
                                      long vol, const double* w, const int* opp, const int* flags, int host_flags,
-                                     double* phi) {
+                                     bool leave_sym, double* phi) {
   using Sh = PairShape<R>;
   const int ts = Sh::ts(n);
   const size_t smem = Sh::smem(n);
@@ -1226,10 +1228,15 @@ static nrcps_status launch_pair_tile(nrcps_context* ctx, const void* psi1, const
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   cudaError_t e =
-      cudaLaunchKernelEx(&cfg, pair_tile_kernel<R>, psi1, psi2, n, vol, w, opp, flags, host_flags, ts, phi);
+      cudaLaunchKernelEx(&cfg, pair_tile_kernel<R>, psi1, psi2, n, vol, w, opp, flags, host_flags, leave_sym ? 1 : 0,
+                         ts, phi);
   ctx->launches++;
   return check_cuda(ctx, e, "pair_tile_kernel launch");
 }
+
+bool pair_sym_supported(int n);  // pair_sym.cu
+nrcps_status pair_sym(nrcps_context* ctx, const void* psi, int n, int nconf, long vol, const double* w, const int* opp,
+                      const int* flags, double* phi);
 
 // props: the table's properties as the caller checked them on the host
 // (pair_table_props), or -1: the device checks them before the tiles.
@@ -1247,8 +1254,15 @@ nrcps_status pair_impl(nrcps_context* ctx, const void* psi1, const void* psi2, i
       flags = ctx->dev_pair_flag;
     }
     if (prec == NRCPS_F64)
-      return launch_pair_tile<double>(ctx, psi1, psi2, n, nconf, vol, w, opp, flags, props, phi);
-    return launch_pair_tile<float>(ctx, psi1, psi2, n, nconf, vol, w, opp, flags, props, phi);
+      return launch_pair_tile<double>(ctx, psi1, psi2, n, nconf, vol, w, opp, flags, props, false, phi);
+    // one set of FP32 orbitals: the packed kernel where the table qualifies;
+    // a table checked on the device decides there which of the two runs
+    const bool one_set = psi1 == psi2 && pair_sym_supported(n);
+    if (one_set && (flags || !props)) {
+      NRCPS_TRY(pair_sym(ctx, psi1, n, nconf, vol, w, opp, flags, phi));
+      if (!flags) return NRCPS_OK;
+    }
+    return launch_pair_tile<float>(ctx, psi1, psi2, n, nconf, vol, w, opp, flags, props, one_set && flags, phi);
   }
   if (prec == NRCPS_F64) pair_kernel<double><<<(unsigned)blocks, 256, 0, ctx->stream>>>(psi1, psi2, n, vol, w, opp, phi);
   else pair_kernel<float><<<(unsigned)blocks, 256, 0, ctx->stream>>>(psi1, psi2, n, vol, w, opp, phi);
