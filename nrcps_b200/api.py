@@ -11,6 +11,7 @@ complex64 are interleaved (re, im), the layout the library expects).
 from __future__ import annotations
 
 import ctypes
+import math
 from dataclasses import dataclass, field as dc_field
 from typing import Optional, Sequence
 
@@ -33,6 +34,16 @@ def _dp(a: np.ndarray):
 
 def _dims(dims) -> np.ndarray:
     return np.ascontiguousarray(np.asarray(dims, dtype=np.int32).reshape(3))
+
+
+_INT3 = ctypes.c_int * 3
+
+
+def _cdims(dims):
+    """Three extents as a C array, for the calls of a time step: no numpy
+    array and ctypes cast on the way (0.5 against 3 us)."""
+    x, y, z = dims
+    return _INT3(x, y, z)
 
 
 def _ptr(t: Optional[torch.Tensor]):
@@ -282,11 +293,11 @@ class Fourier:
         return self.b.shape[0]
 
     def forward(self) -> None:  # FFTW_FORWARD: momentum -> position
-        self.ctx.check(lib().nrcps_fft3d(self.ctx.handle, _ptr(self.b), self.batch_size(), _ip(_dims(self.dims)),
+        self.ctx.check(lib().nrcps_fft3d(self.ctx.handle, _ptr(self.b), self.batch_size(), _cdims(self.dims),
                                          _prec(self.precision), -1), "Fourier::Forward")
 
     def backward(self) -> None:  # FFTW_BACKWARD: position -> momentum
-        self.ctx.check(lib().nrcps_fft3d(self.ctx.handle, _ptr(self.b), self.batch_size(), _ip(_dims(self.dims)),
+        self.ctx.check(lib().nrcps_fft3d(self.ctx.handle, _ptr(self.b), self.batch_size(), _cdims(self.dims),
                                          _prec(self.precision), +1), "Fourier::Backward")
 
     def get(self, n: int) -> torch.Tensor:
@@ -325,7 +336,7 @@ class Potential:
         pass
 
     def evolve(self, b: Fourier) -> None:
-        self.ctx.check(lib().nrcps_potential_evolve(self.ctx.handle, _ptr(b.b), b.batch_size(), _ip(_dims(self.dims)),
+        self.ctx.check(lib().nrcps_potential_evolve(self.ctx.handle, _ptr(b.b), b.batch_size(), _cdims(self.dims),
                                                     _ptr(self.pot), _prec(b.precision)), "Potential::Evolve")
 
 
@@ -343,12 +354,12 @@ class Interaction:
 
     def initialize(self) -> None:
         self.ctx.check(lib().nrcps_interaction_initialize(self.ctx.handle, _ptr(self.lattice.get()), _ptr(self.itab),
-                                                          _ip(_dims(self.dims)), _ptr(self.fld)),
+                                                          _cdims(self.dims), _ptr(self.fld)),
                        "Interaction::Initialize")
 
     def evolve(self, b: Fourier) -> None:
         self.ctx.check(lib().nrcps_interaction_evolve(self.ctx.handle, _ptr(b.b), b.batch_size(),
-                                                      _ip(_dims(self.dims)), _ptr(self.fld), _prec(b.precision)),
+                                                      _cdims(self.dims), _ptr(self.fld), _prec(b.precision)),
                        "Interaction::Evolve")
 
 
@@ -430,14 +441,14 @@ def propagate(psi: torch.Tensor, batch: int, kinv: torch.Tensor, field: torch.Te
     (field_mode 1: Z2 bits, 2: interleaved complex phi, 0: complex fld)."""
     ctx = ctx or default_context()
     dims = tuple(psi.shape[-3:])
-    vol = int(np.prod(dims))
+    vol = math.prod(dims)
     nconf = psi.shape[0] // batch
     pf = C.PositionFactor()
     pf.field_mode, pf.dev_field, pf.bit0 = field_mode, field.data_ptr(), off0
     pf.conf_stride = vol if conf_stride is None else conf_stride
     pf.a, pf.dev_pos = a, (pos.data_ptr() if pos is not None else None)
     prec = C.F64 if psi.dtype == torch.complex128 else C.F32
-    ctx.check(lib().nrcps_propagate(ctx.handle, _ptr(psi), batch, nconf, _ip(_dims(dims)), _ptr(kinv),
+    ctx.check(lib().nrcps_propagate(ctx.handle, _ptr(psi), batch, nconf, _cdims(dims), _ptr(kinv),
                                     ctypes.byref(pf), prec), "propagate")
 
 

@@ -26,6 +26,8 @@
 // (plus the L2-resident k table and field bits).
 #include <cooperative_groups.h>
 
+#include <atomic>
+
 #include "fused.cuh"
 
 namespace cg = cooperative_groups;
@@ -1298,6 +1300,7 @@ static nrcps_status launch_fused(nrcps_context* ctx, const FusedArgs& f, int cta
                           : (KIND == 7 || KIND == 8) ? PullShape<R, L, C, false>::SMEM
                                                      : Sh::SMEM;
   void (*kern)(FusedArgs);
+  int inst = 0;  // which of the kind's kernels
   if constexpr (KIND == 1) kern = fused_step_split_kernel<R, L, C>;
   else if constexpr (KIND == 2) kern = fused_step_bulk_kernel<R, L, C, true>;
   else if constexpr (KIND == 3) kern = fused_step_bulk_kernel<R, L, C, false>;
@@ -1313,23 +1316,20 @@ static nrcps_status launch_fused(nrcps_context* ctx, const FusedArgs& f, int cta
     // position factor) or any other field
     const bool z2 = f.field_mode == 1 && (L * L) % 32 == 0 && (f.pos == nullptr || f.zpos != nullptr);
     kern = z2 ? fused_step_async_kernel<R, L, C, KIND == 12, 1> : fused_step_async_kernel<R, L, C, KIND == 12, 2>;
-    if (!z2) SMEM = AsyncShape<R, L, C, 2>::SMEM;
+    if (!z2) {
+      SMEM = AsyncShape<R, L, C, 2>::SMEM;
+      inst = 1;
+    }
     if constexpr (sizeof(R) == 4) {
       if (f.field_mode == 3) {  // (FP32 only: the host sends mode 3 with FP32 orbitals alone)
         kern = fused_step_async_kernel<R, L, C, KIND == 12, 3>;
         SMEM = AsyncShape<R, L, C, 3>::SMEM;
+        inst = 2;
       }
     }
   }
   else kern = fused_step_kernel<R, L, C>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM);
-  if (e != cudaSuccess) return check_cuda(ctx, e, "fused_step: smem attribute");
-  if (C > 8) {
-    e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-    if (e != cudaSuccess) return check_cuda(ctx, e, "fused_step: cluster attribute");
-  }
   // persistent grid: as many clusters as fit, capped by the work
-  int max_clusters = 0;
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -1342,11 +1342,27 @@ static nrcps_status launch_fused(nrcps_context* ctx, const FusedArgs& f, int cta
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   cfg.gridDim = dim3(C * ctx->sm_count);
-  e = cudaOccupancyMaxActiveClusters(&max_clusters, kern, &cfg);
-  if (e != cudaSuccess || max_clusters <= 0) {
-    cudaGetLastError();
-    max_clusters = ctx->sm_count / C;
-    if (max_clusters < 1) return set_error(ctx, NRCPS_ERR_UNSUPPORTED, "fused_step: cluster of %d does not fit", C);
+  // the attributes and the clusters that fit are asked for once per kernel
+  // (an instance per field class) and device: 3 us of the host on every step
+  static std::atomic<int> fit[3][16];
+  std::atomic<int>* known = ctx->device >= 0 && ctx->device < 16 ? &fit[inst][ctx->device] : nullptr;
+  int max_clusters = known ? known->load(std::memory_order_acquire) : 0;
+  cudaError_t e = cudaSuccess;
+  if (max_clusters == 0) {
+    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM);
+    if (e != cudaSuccess) return check_cuda(ctx, e, "fused_step: smem attribute");
+    if (C > 8) {
+      e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+      if (e != cudaSuccess) return check_cuda(ctx, e, "fused_step: cluster attribute");
+    }
+    e = cudaOccupancyMaxActiveClusters(&max_clusters, kern, &cfg);
+    if (e != cudaSuccess || max_clusters <= 0) {
+      cudaGetLastError();
+      max_clusters = ctx->sm_count / C;
+      if (max_clusters < 1) return set_error(ctx, NRCPS_ERR_UNSUPPORTED, "fused_step: cluster of %d does not fit", C);
+    } else if (known) {
+      known->store(max_clusters, std::memory_order_release);
+    }
   }
   (void)ctas_per_sm_hint;
   long clusters = max_clusters;
