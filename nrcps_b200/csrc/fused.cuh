@@ -30,6 +30,20 @@ struct FusedArgs {
   int stall_test;          // 1: the first wait of CTA 0 of cluster 0 is on an mbarrier nothing arrives on
 };
 
+// x * (wr + i wi)
+template <typename R>
+__device__ __forceinline__ cplx<R> mul_w(cplx<R> x, double wr, double wi) {
+  R rh, rl, ih, il;
+  split<R>(wr, rh, rl);
+  if (wi == 0.0) return scale2<R>(x, rh, rl);  // real weight (Z2, Gaussian, potential): the same value, half the work
+  split<R>(wi, ih, il);
+  // (x.re + i x.im)(wr + i wi) with each real product taken correctly rounded
+  cplx<R> y;
+  y.re = mul2<R>(x.re, rh, rl) - mul2<R>(x.im, ih, il);
+  y.im = mul2<R>(x.re, ih, il) + mul2<R>(x.im, rh, rl);
+  return y;
+}
+
 // x * w for the position-space factor of site `site` (general modes).
 template <typename R>
 __device__ __forceinline__ cplx<R> apply_w_general(const FusedArgs& f, uint64_t kb, int site, cplx<R> x) {
@@ -59,15 +73,56 @@ __device__ __forceinline__ cplx<R> apply_w_general(const FusedArgs& f, uint64_t 
     wr *= p;
     wi *= p;
   }
-  R rh, rl, ih, il;
-  split<R>(wr, rh, rl);
-  if (wi == 0.0) return scale2<R>(x, rh, rl);  // real weight (Z2, Gaussian, potential): the same value, half the work
-  split<R>(wi, ih, il);
-  // (x.re + i x.im)(wr + i wi) with each real product taken correctly rounded
-  cplx<R> y;
-  y.re = mul2<R>(x.re, rh, rl) - mul2<R>(x.im, ih, il);
-  y.im = mul2<R>(x.re, ih, il) + mul2<R>(x.im, rh, rl);
-  return y;
+  return mul_w<R>(x, wr, wi);
+}
+
+// x * w(x) along a pencil of L sites STRIDE apart from `site0`: the values of
+// apply_w_general.  Complex fields are loaded eight sites (four beside FP64
+// pencils, for want of registers) ahead of their use and asked together whether their weights
+// are real: apply_w_general's branch holds each load back until the site
+// before is done, L trips to L2 one after the other.
+template <typename R, int L, int STRIDE>
+__device__ __forceinline__ void apply_w_pencil(const FusedArgs& f, uint64_t kb, int site0, cplx<R>* x) {
+  constexpr int CH = sizeof(R) == 4 ? 8 : 4;
+  static_assert(L % CH == 0, "whole chunks");
+  if (f.field_mode != 0 && f.field_mode != 2) {
+#pragma unroll
+    for (int i = 0; i < L; ++i) x[i] = apply_w_general<R>(f, kb, site0 + i * STRIDE, x[i]);
+    return;
+  }
+  const double2* field = reinterpret_cast<const double2*>(f.field) + kb + (uint64_t)site0;
+  const bool phi = f.field_mode == 2;
+#pragma unroll
+  for (int c = 0; c < L; c += CH) {
+    double2 v[CH];
+#pragma unroll
+    for (int i = 0; i < CH; ++i) v[i] = __ldg(field + (c + i) * STRIDE);
+    bool real = true;
+#pragma unroll
+    for (int i = 0; i < CH; ++i) {
+      if (phi) {
+        v[i].x = (1.0 + f.a * v[i].x) * f.inv_vol;
+        v[i].y = (f.a * v[i].y) * f.inv_vol;
+      }
+      if (f.pos) {
+        const double p = __ldg(f.pos + site0 + (c + i) * STRIDE);
+        v[i].x *= p;
+        v[i].y *= p;
+      }
+      real = real && v[i].y == 0.0;
+    }
+    if (real) {  // (mul_w's product for a real weight)
+#pragma unroll
+      for (int i = 0; i < CH; ++i) {
+        R hi, lo;
+        split<R>(v[i].x, hi, lo);
+        x[c + i] = scale2<R>(x[c + i], hi, lo);
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < CH; ++i) x[c + i] = mul_w<R>(x[c + i], v[i].x, v[i].y);
+    }
+  }
 }
 
 template <typename R, bool PK = false>
@@ -118,7 +173,7 @@ __device__ __forceinline__ cplx<R> scale_w1(cplx<R> x, R w) {
     return cplx<R>{r.x, r.y};
   } else {
     if constexpr (sizeof(R) == 4) return cplx<R>{(R)__fmul_rn((float)x.re, (float)w), (R)__fmul_rn((float)x.im, (float)w)};
-    else return cplx<R>{x.re * w, x.im * w};
+    else return cplx<R>{__dmul_rn(x.re, w), __dmul_rn(x.im, w)};
   }
 }
 

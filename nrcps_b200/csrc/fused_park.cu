@@ -336,8 +336,7 @@ __global__ void __launch_bounds__(PTHREADS, 1) fused_step_park_kernel(FusedArgs 
           x[xx] = cf{__fmul_rn(x[xx].re, w), __fmul_rn(x[xx].im, w)};
         }
       } else {
-#pragma unroll
-        for (int xx = 0; xx < PL; ++xx) x[xx] = apply_w_general<float>(f, kb, site0 + xx * PL * PL, x[xx]);
+        apply_w_pencil<float, PL, PL * PL>(f, kb, site0, x);
       }
       fft::Dft<PL, +1, float>::run(x);
       cf e[PH];

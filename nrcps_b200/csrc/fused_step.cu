@@ -328,8 +328,7 @@ __global__ void __launch_bounds__(PullShape<R, L, C, STAGED>::THREADS, PullShape
           x[xx] = scale_w_zpos<R, PK>(f.zpos, site0 + xx * L * L, up, x[xx]);
         }
       } else {
-#pragma unroll
-        for (int xx = 0; xx < L; ++xx) x[xx] = apply_w_general<R>(f, kb, site0 + xx * L * L, x[xx]);
+        apply_w_pencil<R, L, L * L>(f, kb, site0, x);
       }
       fft::dft<L, +1, R, PK>(x);
 #pragma unroll
@@ -852,8 +851,7 @@ __global__ void __launch_bounds__(BulkShape<R, L, C, STAGED, KSM>::THREADS,
           x[xx] = scale_w_zpos<R, PK>(f.zpos, site0 + xx * L * L, up, x[xx]);
         }
       } else {
-#pragma unroll
-        for (int xx = 0; xx < L; ++xx) x[xx] = apply_w_general<R>(f, kb, site0 + xx * L * L, x[xx]);
+        apply_w_pencil<R, L, L * L>(f, kb, site0, x);
       }
       fft::dft<L, +1, R, PK>(x);
 #pragma unroll
@@ -1220,8 +1218,7 @@ __global__ void __launch_bounds__(PullShape<R, L, C, false>::THREADS, PullShape<
             x[xx] = cplx<R>{(R)__fmul_rn((float)x[xx].re, w), (R)__fmul_rn((float)x[xx].im, w)};
           }
         } else {
-#pragma unroll
-          for (int xx = 0; xx < L; ++xx) x[xx] = apply_w_general<R>(f, kb, site0 + xx * L * L, x[xx]);
+          apply_w_pencil<R, L, L * L>(f, kb, site0, x);
         }
       }
       fft::dft<L, +1, R, PK>(x);
