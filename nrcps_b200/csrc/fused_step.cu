@@ -1393,13 +1393,13 @@ struct FusedVariant {
 static const FusedVariant kVariants[] = {
     {NRCPS_F32, 8, 1, 4, launch_fused<float, 8, 1, 4>},
     {NRCPS_F32, 8, 1, 0, launch_fused<float, 8, 1>},
+    {NRCPS_F32, 16, 2, 11, launch_fused<float, 16, 2, 11>},
     {NRCPS_F32, 16, 1, 0, launch_fused<float, 16, 1>},
     {NRCPS_F32, 16, 1, 4, launch_fused<float, 16, 1, 4>},
     {NRCPS_F32, 16, 2, 2, launch_fused<float, 16, 2, 2>},
     {NRCPS_F32, 16, 2, 9, launch_fused<float, 16, 2, 9>},
     {NRCPS_F32, 16, 2, 10, launch_fused<float, 16, 2, 10>},
     {NRCPS_F32, 16, 2, 0, launch_fused<float, 16, 2>},
-    {NRCPS_F32, 16, 2, 11, launch_fused<float, 16, 2, 11>},
     {NRCPS_F32, 16, 1, 1, launch_fused<float, 16, 1, 1>},
     {NRCPS_F32, 24, 3, 5, launch_fused<float, 24, 3, 5>},
     {NRCPS_F32, 24, 4, 4, launch_fused<float, 24, 4, 4>},
@@ -1451,6 +1451,15 @@ static const FusedVariant kVariants[] = {
 };
 static const int kNumVariants = sizeof(kVariants) / sizeof(kVariants[0]);
 
+nrcps_status fused_park_step(nrcps_context* ctx, const FusedArgs& f);  // fused_park.cu
+int fused_one_slots(const nrcps_context* ctx, nrcps_precision prec, int L);  // fused_one.cu
+nrcps_status fused_one_step(nrcps_context* ctx, nrcps_precision prec, const FusedArgs& f);
+
+// Orbitals in flight in the kernel that holds one in a CTA; 0: there is none.
+static long whole_slots(const nrcps_context* ctx, nrcps_precision prec, int L) {
+  return prec == NRCPS_F32 && L == 32 ? ctx->sm_count : fused_one_slots(ctx, prec, L);
+}
+
 // Autotuned choice per (device, precision, L): index into kVariants, -1 unset.
 static int g_choice[16][2][64];
 static bool g_choice_init = false;
@@ -1498,6 +1507,16 @@ __global__ void autotune_unit_kin_kernel(void* kin, long V, int fp64) {
 nrcps_status fused_autotune(nrcps_context* ctx, nrcps_precision prec, int L, int* chosen_cluster) {
   init_choices();
   int dev = ctx->device & 15;
+  if (L < 64 && g_choice[dev][prec][L] < 0 && whole_slots(ctx, prec, L)) {
+    // Large batches run an orbital per CTA; a variant serves the batches below
+    // and is the first listed, which is measured best there: L = 16, FP32, 168
+    // orbitals: kind 11, cluster 2 13.4 us a step, kind 0, cluster 1 17.5 (at
+    // 8192 orbitals, which would be timed here, 214 and 164).  All three listed
+    // first are scalar kinds, whose arithmetic the whole-orbital kernels have:
+    // results do not depend on the size of the batch.
+    for (int i = 0; i < kNumVariants && g_choice[dev][prec][L] < 0; ++i)
+      if (kVariants[i].prec == prec && kVariants[i].L == L) g_choice[dev][prec][L] = i;
+  }
   if (L < 64 && g_choice[dev][prec][L] >= 0) {
     if (chosen_cluster)
       *chosen_cluster = kVariants[g_choice[dev][prec][L]].C * (kVariants[g_choice[dev][prec][L]].kind == 1 ? -1 : 1);
@@ -1565,11 +1584,6 @@ nrcps_status fused_autotune(nrcps_context* ctx, nrcps_precision prec, int L, int
   for (int i = 0; i < kNumVariants; ++i) {
     round_ms[i] = 1e30f;
     ok[i] = kVariants[i].prec == prec && kVariants[i].L == L;
-    // FP32 at L = 32: small batches run the variant chosen here and large
-    // ones the one-SM kernel, whose arithmetic is the scalar kinds': keep to
-    // those, so that results do not depend on the size of the batch
-    const int k = kVariants[i].kind;
-    if (prec == NRCPS_F32 && L == 32 && !(k == 0 || k == 2 || k == 3 || k == 7 || k == 10 || k == 11)) ok[i] = false;
   }
   for (int round = 0; round < 3; ++round) {
     for (int i = 0; i < kNumVariants; ++i) {
@@ -1633,25 +1647,34 @@ static int fused_pick(nrcps_context* ctx, nrcps_precision prec, int L, int clust
   return pick;
 }
 
-nrcps_status fused_park_step(nrcps_context* ctx, const FusedArgs& f);  // fused_park.cu
 
-// Whether a step of n_orb orbitals runs in the one-SM kernel (FP32, L = 32,
-// no variant forced).  It takes an SM per orbital, 148 at a time (26 us each
-// at 19456 orbitals, 0.182 us per orbital against 0.246 for kind 11, cluster
-// 8, which spreads an orbital over 8 CTAs, 74 at a time): it pays where its
-// last wave is not mostly empty.  Measured, one-SM against cluster kernel: 57
-// orbitals 32 / 26 us, 95 35 / 37, 152 61 / 50, 190 61 / 58, 304 87 / 85, 988
-// 224 / 258, 19456 3544 / 4778.
-static bool fused_park_pays(nrcps_context* ctx, nrcps_precision prec, int L, int cluster, long n_orb) {
-  if (prec != NRCPS_F32 || L != 32 || cluster > 0 || ctx->fused_split >= 0 || ctx->fused_kind >= 0) return false;
-  const long sm = ctx->sm_count, waves = (n_orb + sm - 1) / sm;
-  return 3 * n_orb > 2 * waves * sm;
+// The kind (13, 14 or 0) of the kernel that holds an orbital in one CTA and
+// runs a step of n_orb orbitals where no variant is forced: 13 half parked in
+// tensor memory (FP32, L = 32), 14 in shared memory (L = 16).  They take
+// an orbital per CTA, `slots` at a time (kind 13: 26 us each at 19456
+// orbitals, 0.182 us per orbital against 0.246 for kind 11, cluster 8, which
+// spreads an orbital over 8 CTAs, 74 at a time).  Kind 13 pays where its last
+// wave is not mostly empty, kind 14, which has several CTAs per SM, from half a
+// wave on.  Measured, kind 13 against kind 11: 57 orbitals 32 / 26
+// us, 95 35 / 37, 152 61 / 50, 190 61 / 58, 304 87 / 85, 988 224 / 258, 19456
+// 3544 / 4778; kind 14, FP64 (444 slots) against kind 0, cluster 2: 300
+// orbitals 17 / 20 us, 444 17 / 23, 600 25 / 31, 3500 131 / 161; FP32 (888
+// slots) against kind 11, cluster 2: 600 18 / 27, 2100 42 / 53.
+static int fused_whole_kind(nrcps_context* ctx, nrcps_precision prec, int L, int cluster, long n_orb) {
+  if (cluster > 0 || ctx->fused_split >= 0 || ctx->fused_kind >= 0) return 0;
+  const bool park = L == 32;
+  const long slots = whole_slots(ctx, prec, L);
+  if (slots == 0) return 0;
+  if (!park) return 2 * n_orb > slots ? 14 : 0;
+  const long waves = (n_orb + slots - 1) / slots;
+  return 3 * n_orb > 2 * waves * slots ? 13 : 0;
 }
 
 nrcps_status fused_choice(nrcps_context* ctx, nrcps_precision prec, int L, int* kind, int* cluster) {
   const int d[3] = {L, L, L};
-  if (ctx->fused_enabled && fused_park_pays(ctx, prec, L, ctx->fused_cluster, ctx->sm_count)) {
-    *kind = 13;
+  const int whole = ctx->fused_enabled ? fused_whole_kind(ctx, prec, L, ctx->fused_cluster, 1L << 20) : 0;
+  if (whole) {  // (large batches)
+    *kind = whole;
     *cluster = 1;
     return NRCPS_OK;
   }
@@ -1694,7 +1717,10 @@ nrcps_status fused_step(nrcps_context* ctx, void* psi, int batch, int nconf, con
   f.wait_ns = ctx->fused_wait_ns;
   f.stall_test = ctx->fused_stall_test;
   if (f.n_orb_total == 0) return NRCPS_OK;
-  if (fused_park_pays(ctx, prec, d[0], cluster, f.n_orb_total)) return fused_park_step(ctx, f);
+  switch (fused_whole_kind(ctx, prec, d[0], cluster, f.n_orb_total)) {
+    case 13: return fused_park_step(ctx, f);
+    case 14: return fused_one_step(ctx, prec, f);
+  }
   const int pick = fused_pick(ctx, prec, d[0], cluster);
   if (pick < 0)
     return set_error(ctx, NRCPS_ERR_UNSUPPORTED, "no fused variant with cluster size %d, split %d, kind %d",
