@@ -146,7 +146,8 @@ inline long vol_of(const int dims[3]) { return (long)dims[0] * dims[1] * dims[2]
 // tensor-core overlap (overlap_tc.cu)
 bool overlap_tc_supported(long vol, int ns, int nt, int nconf);
 size_t overlap_tc_split_bytes(int ns, long vol);
-nrcps_status overlap_tc_prepare(nrcps_context* ctx, const double* src, int ns, long vol, float* split);
+nrcps_status overlap_tc_prepare(nrcps_context* ctx, const double* src, int ns, long vol, int nt, int nconf,
+                                float* split);
 nrcps_status overlap_tc(nrcps_context* ctx, const float* split, int ns, const void* psi, int nt, int nconf, long vol,
                         double* S);
 

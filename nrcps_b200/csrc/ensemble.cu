@@ -277,7 +277,7 @@ extern "C" nrcps_status nrcps_ensemble_create(nrcps_context* ctx, const nrcps_jo
       return fail(st);
     if (job->precision == NRCPS_F32 && ctx->overlap_tc && overlap_tc_supported(V, N, N, nc)) {
       if ((st = dalloc(ctx, (char**)&e->src_split, overlap_tc_split_bytes(N, V))) ||
-          (st = overlap_tc_prepare(ctx, e->src, N, V, e->src_split)))
+          (st = overlap_tc_prepare(ctx, e->src, N, V, N, nc, e->src_split)))
         return fail(st);
     } else if ((st = overlap_reserve(ctx))) {  // the time loop is captured: nothing is allocated there
       return fail(st);
@@ -399,7 +399,7 @@ extern "C" nrcps_status nrcps_ensemble_set_sources(nrcps_ensemble* e, const doub
   NRCPS_REQUIRE(ctx, sources, "nrcps_ensemble_set_sources: dense-source ensemble needs sources");
   NRCPS_TRY(check_cuda(ctx, cudaMemcpyAsync(e->src, sources, 16 * (size_t)e->N * e->vol, cudaMemcpyHostToDevice,
                                             ctx->stream), "set_sources: copy sources"));
-  if (e->src_split) NRCPS_TRY(overlap_tc_prepare(ctx, e->src, e->N, e->vol, e->src_split));
+  if (e->src_split) NRCPS_TRY(overlap_tc_prepare(ctx, e->src, e->N, e->vol, e->N, e->job.n_conf, e->src_split));
   return NRCPS_OK;
 }
 

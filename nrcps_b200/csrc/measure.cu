@@ -1293,7 +1293,7 @@ extern "C" nrcps_status nrcps_overlap(nrcps_context* ctx, const double* dev_src,
       NRCPS_TRY(check_cuda(ctx, cudaMalloc(&ctx->tc_split, need), "cudaMalloc(overlap split)"));
       ctx->tc_split_bytes = need;
     }
-    NRCPS_TRY(overlap_tc_prepare(ctx, dev_src, ns, vol, (float*)ctx->tc_split));
+    NRCPS_TRY(overlap_tc_prepare(ctx, dev_src, ns, vol, nt, nconf, (float*)ctx->tc_split));
     return overlap_tc(ctx, (const float*)ctx->tc_split, ns, dev_psi, nt, nconf, vol, dev_S);
   }
   return overlap_impl(ctx, dev_src, ns, dev_psi, nt, nconf, vol, prec, dev_S);

@@ -458,8 +458,19 @@ size_t overlap_tc_split_bytes(int ns, long vol) { return sizeof(float) * 2 * (si
 
 // Builds the hi / lo A operands of every source block into `split`
 // (overlap_tc_split_bytes(ns, vol) bytes): block b (sources 32 b ...) at
-// float offset 2 * 2 * 32 b * 2V.
-nrcps_status overlap_tc_prepare(nrcps_context* ctx, const double* src, int ns, long vol, float* split) {
+// float offset 2 * 2 * 32 b * 2V; for overlap_tc calls of nconf configurations
+// of nt orbitals.
+//
+// Where overlap_few.cu's CUDA-core kernel is the faster one, both calls go
+// there instead; it takes the sources as plain FP32 (a quarter of the bytes).
+bool overlap_few_pays(int ns, int nt, int nconf, long vol);
+nrcps_status overlap_few_prepare(nrcps_context* ctx, const double* src, int ns, long vol, float* out);
+nrcps_status overlap_few(nrcps_context* ctx, const float* src, int ns, const void* psi, int nt, int nconf, long vol,
+                         double* S);
+
+nrcps_status overlap_tc_prepare(nrcps_context* ctx, const double* src, int ns, long vol, int nt, int nconf,
+                                float* split) {
+  if (overlap_few_pays(ns, nt, nconf, vol)) return overlap_few_prepare(ctx, src, ns, vol, split);
   const long K = 2 * vol;
   for (int sb = 0; sb < ns; sb += tc::MAX_NS_BLOCK) {
     const int nsb = ns - sb < tc::MAX_NS_BLOCK ? ns - sb : tc::MAX_NS_BLOCK;
@@ -479,6 +490,7 @@ nrcps_status overlap_tc(nrcps_context* ctx, const float* split, int ns, const vo
   const long K = 2 * vol;
   const int n_rows = nt * nconf;
   if (n_rows == 0 || ns == 0) return NRCPS_OK;
+  if (overlap_few_pays(ns, nt, nconf, vol)) return overlap_few(ctx, split, ns, psi, nt, nconf, vol, S);
   static bool attr_set[16] = {false};
   if (!attr_set[ctx->device & 15]) {
     NRCPS_TRY(check_cuda(ctx,

@@ -34,7 +34,7 @@
 // configurations: 0.81 ms against 1.20.
 #include <cooperative_groups.h>
 
-#include "common.cuh"
+#include "lane_sums.cuh"
 
 namespace nrcps {
 namespace cg = cooperative_groups;
@@ -70,32 +70,10 @@ __device__ __forceinline__ void copy8(void* dst, const void* src, bool take) {
                : "memory");
 }
 
-constexpr int SLEVELS = 5;      // levels of the FP32 tree
-constexpr int skept(int values) { return (values > 32 ? 64 : 32) >> SLEVELS; }  // values a lane takes into FP64
-
-// v[0 .. N): the sums over the 2^SLEVELS lanes that differ in the upper lane
-// bits; of the (padded) values each keeps a run of skept(N), in v[0 ..)
-template <int N>
-__device__ __forceinline__ void reduce_scatter(float (&v)[N], int lane) {
-  constexpr int FULL = N > 32 ? 64 : 32;
-#pragma unroll
-  for (int l = 0; l < SLEVELS; ++l) {
-    const int h = FULL >> (l + 1), bit = 16 >> l;
-    const bool up = lane & bit;
-#pragma unroll
-    for (int k = 0; k < h; ++k) {
-      if (k >= N) continue;
-      const float hi = k + h < N ? v[k + h] : 0.f;  // (entries past N are zeros)
-      const float keep = up ? hi : v[k], send = up ? v[k] : hi;
-      v[k] = keep + __shfl_xor_sync(0xffffffffu, send, bit);
-    }
-  }
-}
-
 // A warp's block: all 25 entries, or the 15 of the triangle (DIAG).
 struct SymAcc {
   float2 P[SB * SB], Q[SB * SB];
-  double sum[skept(2 * SB * SB)];
+  double sum[lane_share(2 * SB * SB)];
   int count;
   template <bool DIAG>
   static __host__ __device__ constexpr int entries() {
@@ -136,7 +114,7 @@ struct SymAcc {
     }
     reduce_scatter<2 * entries<DIAG>()>(v, lane);
 #pragma unroll
-    for (int k = 0; k < skept(2 * entries<DIAG>()); ++k) sum[k] += (double)v[k];
+    for (int k = 0; k < lane_share(2 * entries<DIAG>()); ++k) sum[k] += (double)v[k];
     clear();
   }
 };
@@ -305,16 +283,8 @@ __global__ void __launch_bounds__(SymShape<NB>::THREADS, SymShape<NB>::CTAS)
   __syncthreads();
   // every warp's sums over the stages, then the cluster's CTAs in rank order
   double* red = reinterpret_cast<double*>(ssm);  // [WARPS][64]
-  // (the lanes that hold the same run add theirs up in order)
-  constexpr int RUNS = 1 << SLEVELS;
-  const int kept = skept(diag ? 2 * SymAcc::entries<true>() : 2 * SymAcc::entries<false>());
-#pragma unroll
-  for (int k = 0; k < skept(2 * SB * SB); ++k) {
-    double v = acc.sum[k];
-#pragma unroll
-    for (int b = 1; b < 32 / RUNS; b <<= 1) v += __shfl_xor_sync(0xffffffffu, v, b);
-    if (k < kept && lane % (32 / RUNS) == 0) red[warp * 64 + lane / (32 / RUNS) * kept + k] = v;
-  }
+  const int share = lane_share(2 * (diag ? SymAcc::entries<true>() : SymAcc::entries<false>()));
+  for (int k = 0; k < share; ++k) red[warp * 64 + share * lane + k] = acc.sum[k];
   cluster.sync();
   for (int e = rank * Sh::THREADS + threadIdx.x; e < 2 * n * n; e += split * Sh::THREADS) {
     const int s = e / 2 / n, t = e / 2 % n, c = e & 1;
