@@ -142,16 +142,19 @@ const char *nrcps_version(void);
 nrcps_status nrcps_set_option(nrcps_context *ctx, const char *name, long value);
 /* Times every fused-kernel variant (cluster size, lane split) for (prec, L)
  * on this device and keeps the fastest for later calls; *cluster receives
- * its cluster size, negated for the lane-split variants (may be NULL). */
+ * its cluster size, negated for the lane-split variants (may be NULL).  Where
+ * large batches run an orbital per CTA (kinds 13 and 14 of
+ * nrcps_fused_choice), a variant serves small batches only and is fixed:
+ * nothing is timed. */
 nrcps_status nrcps_autotune(nrcps_context *ctx, nrcps_precision prec, int L, int *cluster);
 /* The fused-kernel variant that nrcps_propagate uses for (prec, L^3) on this
  * context's device under its current options (no counterpart in the
  * reference; it names the kernel behind a measurement): *kind (0..12, see
  * "fused.kind") and *cluster (CTAs per cluster); both -1 when no fused
- * variant serves the shape.  (13, 1) names the kernel that holds an orbital in
- * one SM (FP32, L = 32): it runs where no variant is forced and the batch
- * fills the device; smaller batches run the autotuned variant, with the same
- * results.  Tunes nothing. */
+ * variant serves the shape.  (13, 1) and (14, 1) name the kernels that hold an
+ * orbital in one SM (FP32, L = 32) and in one CTA (L = 16): they run where no
+ * variant is forced and the batch fills the device, or half of it; smaller
+ * batches run a variant, with the same results.  Tunes nothing. */
 nrcps_status nrcps_fused_choice(nrcps_context *ctx, nrcps_precision prec, int L, int *kind, int *cluster);
 
 /* ----------------------------------------------------- host-side tables
