@@ -23,10 +23,10 @@ struct PencilGeom {
   long stride;        // site stride along the pencil
 };
 
-enum PencilOp { OP_NONE = 0, OP_PRE_MUL = 1, OP_POST_MUL = 2, OP_MID_FIELD = 3 };
+enum PencilOp { OP_NONE = 0, OP_PRE_MUL = 1, OP_POST_MUL = 2, OP_MID_FIELD = 3, OP_MID_REAL = 4 };
 
 struct FieldArgs {
-  int mode;              // 0 complex fld, 1 Z2 bits, 2 interleaved complex phi, 3 real FP32 weights, 4 none (pos alone)
+  int mode;              // 0 complex fld, 1 Z2 bits, 2 interleaved complex phi, 3 real FP32 weights
   const void* field;
   uint64_t bit0;         // element (mode 0/2) or bit (mode 1) offset of configuration 0
   uint64_t conf_stride;  // elements or bits between configurations
@@ -37,18 +37,18 @@ struct FieldArgs {
   int orbs_per_conf;
 };
 
+// w_plus, w_minus: (1 +- a) / V of a Z2 field, which would be an FP64 division
+// per site
 template <typename R>
-__device__ __forceinline__ cplx<R> field_factor(const FieldArgs& f, long conf, long site) {
+__device__ __forceinline__ cplx<R> field_factor(const FieldArgs& f, R w_plus, R w_minus, long conf, long site) {
   cplx<R> w;
-  if (f.mode == 4) return cplx<R>{(R)f.pos[site], (R)0};
   const uint64_t k = f.bit0 + (f.conf_base ? f.conf_base[conf] : (uint64_t)conf * f.conf_stride) + (uint64_t)site;
   if (f.mode == 0) {
     double2 v = reinterpret_cast<const double2*>(f.field)[k];
     w = cplx<R>{(R)v.x, (R)v.y};
   } else if (f.mode == 1) {
     uint32_t word = reinterpret_cast<const uint32_t*>(f.field)[k >> 5];
-    double phi = ((word >> (k & 31)) & 1u) ? 1.0 : -1.0;
-    w = cplx<R>{(R)((1.0 + f.a * phi) / f.vol), (R)0};
+    w = cplx<R>{((word >> (k & 31)) & 1u) ? w_plus : w_minus, (R)0};
   } else if (f.mode == 3) {
     w = cplx<R>{(R)reinterpret_cast<const float*>(f.field)[k], (R)0};
   } else {
@@ -66,6 +66,11 @@ __device__ __forceinline__ cplx<R> field_factor(const FieldArgs& f, long conf, l
 template <typename R, int N, int SIGN, int OP>
 __global__ void __launch_bounds__(128) pencil_kernel(void* data, long total, PencilGeom g,
                                                      const double* table, FieldArgs f) {
+  [[maybe_unused]] R w_plus = 0, w_minus = 0;
+  if constexpr (OP == OP_MID_FIELD) {
+    w_plus = (R)((1.0 + f.a) / f.vol);
+    w_minus = (R)((1.0 - f.a) / f.vol);
+  }
   for (long p = (long)blockIdx.x * blockDim.x + threadIdx.x; p < total; p += (long)gridDim.x * blockDim.x) {
     const long b = p / g.npencils;
     const long r = p - b * g.npencils;
@@ -86,7 +91,15 @@ __global__ void __launch_bounds__(128) pencil_kernel(void* data, long total, Pen
     if constexpr (OP == OP_MID_FIELD) {
       const long conf = b / f.orbs_per_conf;
 #pragma unroll
-      for (int j = 0; j < N; ++j) x[j] = cmul(field_factor<R>(f, conf, site0 + j * g.stride), x[j]);
+      for (int j = 0; j < N; ++j) x[j] = cmul(field_factor<R>(f, w_plus, w_minus, conf, site0 + j * g.stride), x[j]);
+      fft::Dft<N, -SIGN, R>::run(x);
+    }
+    if constexpr (OP == OP_MID_REAL) {
+#pragma unroll
+      for (int j = 0; j < N; ++j) {
+        const R k = (R)table[site0 + j * g.stride];
+        x[j] = cplx<R>{x[j].re * k, x[j].im * k};
+      }
       fft::Dft<N, -SIGN, R>::run(x);
     }
     if constexpr (OP == OP_POST_MUL) {
@@ -313,16 +326,15 @@ static nrcps_status evolve_any(nrcps_context* ctx, void* psi, int batch, const i
   // occupancy wins, 2000 orbitals of 12^3 98 / 90 us)
   if (evolve_fits(prec, d) && batch <= 6 * ctx->sm_count) return evolve_step(ctx, psi, batch, d, w, w_complex, prec);
   FieldArgs none{}, f{};
-  f.mode = w_complex ? 0 : 4;
-  f.field = w;
-  f.pos = w_complex ? nullptr : w;
+  f.field = w;  // (mode 0)
   f.vol = (double)vol_of(d);
   f.orbs_per_conf = batch;
   auto passes = [&](auto zero) {
     using R = decltype(zero);
     NRCPS_TRY((launch_axis<R, -1, OP_NONE>(ctx, psi, batch, d, 2, nullptr, none)));
     NRCPS_TRY((launch_axis<R, -1, OP_NONE>(ctx, psi, batch, d, 1, nullptr, none)));
-    NRCPS_TRY((launch_axis<R, -1, OP_MID_FIELD>(ctx, psi, batch, d, 0, nullptr, f)));
+    if (w_complex) NRCPS_TRY((launch_axis<R, -1, OP_MID_FIELD>(ctx, psi, batch, d, 0, nullptr, f)));
+    else NRCPS_TRY((launch_axis<R, -1, OP_MID_REAL>(ctx, psi, batch, d, 0, w, none)));
     NRCPS_TRY((launch_axis<R, +1, OP_NONE>(ctx, psi, batch, d, 1, nullptr, none)));
     return launch_axis<R, +1, OP_NONE>(ctx, psi, batch, d, 2, nullptr, none);
   };
@@ -383,15 +395,11 @@ extern "C" nrcps_status nrcps_interaction_initialize(nrcps_context* ctx, const d
   copy_kernel<<<grid, 256, 0, ctx->stream>>>(dev_fld, dev_lat, 2 * vol);
   ctx->launches++;
   NRCPS_TRY(check_launch(ctx, "copy_kernel"));
-  FieldArgs none{}, f{};
-  f.mode = 4;
-  f.pos = dev_itab;
-  f.vol = (double)vol;
-  f.orbs_per_conf = 1;
+  FieldArgs none{};
   NRCPS_TRY((launch_axis<double, +1, OP_NONE>(ctx, dev_fld, 1, dims, 2, nullptr, none)));
   NRCPS_TRY((launch_axis<double, +1, OP_NONE>(ctx, dev_fld, 1, dims, 1, nullptr, none)));
   if (dims[0] < 48) {
-    NRCPS_TRY((launch_axis<double, +1, OP_MID_FIELD>(ctx, dev_fld, 1, dims, 0, nullptr, f)));
+    NRCPS_TRY((launch_axis<double, +1, OP_MID_REAL>(ctx, dev_fld, 1, dims, 0, dev_itab, none)));
   } else {  // (two FP64 transforms of 48 in one thread spill; few pencils hide it badly: 70 us against 66)
     NRCPS_TRY((launch_axis<double, +1, OP_NONE>(ctx, dev_fld, 1, dims, 0, nullptr, none)));
     mul_real_kernel<<<grid_for(vol, 256), 256, 0, ctx->stream>>>(dev_fld, vol, dev_itab);
