@@ -1647,6 +1647,12 @@ static int fused_pick(nrcps_context* ctx, nrcps_precision prec, int L, int clust
   return pick;
 }
 
+// Whether a fused step of (prec, d) runs under the context's options, a forced
+// variant among them: asked before the first launch by callers that have
+// another path (a psi off 16 bytes is the caller's to look at).
+bool fused_admits(nrcps_context* ctx, nrcps_precision prec, const int d[3]) {
+  return ctx->fused_enabled && fused_supported(prec, d) && fused_pick(ctx, prec, d[0], ctx->fused_cluster) >= 0;
+}
 
 // The kind (13, 14 or 0) of the kernel that holds an orbital in one CTA and
 // runs a step of n_orb orbitals where no variant is forced: 13 half parked in

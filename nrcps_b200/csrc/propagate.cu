@@ -254,6 +254,7 @@ extern "C" nrcps_status nrcps_kinetic_evolve(nrcps_context* ctx, void* psi, int 
 
 namespace nrcps {
 bool fused_supported(nrcps_precision prec, const int d[3]);
+bool fused_admits(nrcps_context* ctx, nrcps_precision prec, const int d[3]);
 nrcps_status fused_step(nrcps_context* ctx, void* psi, int batch, int nconf, const int d[3], const void* kin_table,
                         nrcps_precision prec, const nrcps_position_factor* w, int cluster, const void* zpos);
 bool evolve_fits(nrcps_precision prec, const int d[3]);  // evolve.cu
@@ -301,7 +302,7 @@ static const double* unit_table(nrcps_context* ctx, int L) {
 // B[w . F[psi]]; NRCPS_ERR_UNSUPPORTED where it does not serve.
 static nrcps_status evolve_fused(nrcps_context* ctx, void* psi, int batch, const int d[3], const double* w,
                                  bool w_complex, nrcps_precision prec) {
-  if (!ctx->fused_enabled || !fused_supported(prec, d)) return NRCPS_ERR_UNSUPPORTED;
+  if (!fused_admits(ctx, prec, d)) return NRCPS_ERR_UNSUPPORTED;
   const long V = vol_of(d);
   const double* unit = unit_table(ctx, d[0]);
   if (!unit) return NRCPS_ERR_UNSUPPORTED;
@@ -378,9 +379,10 @@ extern "C" nrcps_status nrcps_interaction_initialize(nrcps_context* ctx, const d
   NRCPS_TRY(check_dims(ctx, dims));
   const long vol = vol_of(dims);
   // one field: a CTA does it up to 8192 sites, a cluster does a larger cube
-  // (as conj(B[c F[conj(phi)]]), c being real), pencil passes the rest
+  // (as conj(B[c F[conj(phi)]]), c being real), pencil passes the rest, and
+  // all where the context's options force a variant that FP64 does not have
   if (vol <= 8192 && evolve_fits(NRCPS_F64, dims)) return evolve_initialize(ctx, dev_lat, dev_itab, dims, dev_fld);
-  if (ctx->fused_enabled && fused_supported(NRCPS_F64, dims) && unit_table(ctx, dims[0]) &&
+  if (fused_admits(ctx, NRCPS_F64, dims) && unit_table(ctx, dims[0]) &&
       (reinterpret_cast<uintptr_t>(dev_fld) & 15) == 0 && (reinterpret_cast<uintptr_t>(dev_lat) & 15) == 0) {
     conj_kernel<<<grid_for(vol, 256), 256, 0, ctx->stream>>>(reinterpret_cast<double2*>(dev_fld),
                                                              reinterpret_cast<const double2*>(dev_lat), vol);
