@@ -380,10 +380,12 @@ extern "C" nrcps_status nrcps_interaction_initialize(nrcps_context* ctx, const d
   const long vol = vol_of(dims);
   // one field: a CTA does it up to 8192 sites, a cluster does a larger cube
   // (as conj(B[c F[conj(phi)]]), c being real), pencil passes the rest, and
-  // all where the context's options force a variant that FP64 does not have
-  if (vol <= 8192 && evolve_fits(NRCPS_F64, dims)) return evolve_initialize(ctx, dev_lat, dev_itab, dims, dev_fld);
-  if (fused_admits(ctx, NRCPS_F64, dims) && unit_table(ctx, dims[0]) &&
-      (reinterpret_cast<uintptr_t>(dev_fld) & 15) == 0 && (reinterpret_cast<uintptr_t>(dev_lat) & 15) == 0) {
+  // all where the context's options force a variant that FP64 does not have or
+  // the field starts on 8 bytes (copy_kernel reads doubles)
+  const bool aligned = ((reinterpret_cast<uintptr_t>(dev_fld) | reinterpret_cast<uintptr_t>(dev_lat)) & 15) == 0;
+  if (aligned && vol <= 8192 && evolve_fits(NRCPS_F64, dims))
+    return evolve_initialize(ctx, dev_lat, dev_itab, dims, dev_fld);
+  if (aligned && fused_admits(ctx, NRCPS_F64, dims) && unit_table(ctx, dims[0])) {
     conj_kernel<<<grid_for(vol, 256), 256, 0, ctx->stream>>>(reinterpret_cast<double2*>(dev_fld),
                                                              reinterpret_cast<const double2*>(dev_lat), vol);
     ctx->launches++;

@@ -51,3 +51,21 @@ def test_initialize_and_evolve_under_forced_variants(L, options):
     assert _close(b, _back(c * _fft(psi)), 1e-14)
     assert lib().nrcps_last_error(ctx.handle) in (b"", None)
     ctx.close()
+
+
+@pytest.mark.parametrize("dims", [(8, 8, 8), (4, 6, 12), (24, 24, 24)])
+def test_initialize_from_a_field_on_eight_bytes(dims):
+    """A field that starts at an odd double of its buffer: the same values."""
+    import nrcps_b200 as nb
+    from nrcps_b200.api import lib, _ip, _dims, _ptr
+    ctx = nb.default_context()
+    d3, V = _ip(_dims(dims)), int(np.prod(dims))
+    g = torch.Generator(device=ctx.device).manual_seed(V)
+    room = torch.randn(2 * V + 1, dtype=torch.float64, device=ctx.device, generator=g)
+    lat = room[1:]
+    assert lat.data_ptr() % 16 == 8
+    c = torch.rand(dims, dtype=torch.float64, device=ctx.device, generator=g) / V
+    out = torch.empty(dims, dtype=torch.complex128, device=ctx.device)
+    ctx.check(lib().nrcps_interaction_initialize(ctx.handle, _ptr(lat), _ptr(c), d3, _ptr(out)))
+    phi = torch.view_as_complex(lat.clone().view(*dims, 2))
+    assert _close(out, (1 + _fft(c * _back(phi))) / V, 1e-14)
