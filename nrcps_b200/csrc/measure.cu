@@ -1049,13 +1049,14 @@ static int warp_lu_warps(int N) {
 }
 
 // Leading-minor determinants by a warp per minor (N <= 64, no scratch): rows in
-// registers up to N = 32, the minor in shared memory above.
+// registers up to N = 32 (read 16 bytes at a time: matrices that start on 16),
+// the minor in shared memory otherwise.
 nrcps_status slater_dets_warp(nrcps_context* ctx, const double* S, const double* psi1, int N, int nconf, int mode,
                               int log_det, double* out, long out_conf_stride, long out_offset) {
   const int nmeas = mode ? 2 * N : N;
   const long total = (long)nconf * nmeas;
   if (total == 0) return NRCPS_OK;
-  if (N <= kRowLuMax) {
+  if (N <= kRowLuMax && ((reinterpret_cast<uintptr_t>(S) | reinterpret_cast<uintptr_t>(psi1)) & 15) == 0) {
     const long blocks = minor_blocks(nconf, mode, 16, N, 1) + minor_blocks(nconf, mode, 8, N < 16 ? N : 16, 2) +
                         minor_blocks(nconf, mode, 0, N < 8 ? N : 8, 4);
     auto launch = [&](auto kern) {
