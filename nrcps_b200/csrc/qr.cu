@@ -171,9 +171,16 @@ __global__ void __launch_bounds__(CHOL_THREADS) chol_inv_kernel(double* __restri
                                                                 double* __restrict__ logR, int f32_apply) {
   extern __shared__ double2 cm[];  // [N][N]
   const long c = blockIdx.x;
-  double2* g = reinterpret_cast<double2*>(G) + c * N * N;
+  double* g = G + 2 * c * N * N;  // (the caller's work buffer: doubles, not on 16 bytes of need)
+  auto write_back = [&]() {
+    for (int e = threadIdx.x; e < N * N; e += CHOL_THREADS)
+      if (e / N <= e % N) {
+        g[2 * e] = cm[e].x;
+        g[2 * e + 1] = cm[e].y;
+      }
+  };
   for (int e = threadIdx.x; e < N * N; e += CHOL_THREADS)
-    if (e / N <= e % N) cm[e] = g[e];
+    if (e / N <= e % N) cm[e] = make_double2(g[2 * e], g[2 * e + 1]);
   __syncthreads();
   bool ok = true;
   for (int k = 0; k < N; ++k) {
@@ -207,8 +214,7 @@ __global__ void __launch_bounds__(CHOL_THREADS) chol_inv_kernel(double* __restri
     __syncthreads();
   }
   if (!ok) {
-    for (int e = threadIdx.x; e < N * N; e += CHOL_THREADS)
-      if (e / N <= e % N) g[e] = cm[e];
+    write_back();
     for (int i = threadIdx.x; i < N; i += CHOL_THREADS) logR[c * N + i] = nan("");
     return;
   }
@@ -235,8 +241,7 @@ __global__ void __launch_bounds__(CHOL_THREADS) chol_inv_kernel(double* __restri
   }
   if (f32_apply)
     for (int i = threadIdx.x; i < N; i += CHOL_THREADS) logR[c * N + i] -= log((double)(float)cm[i * N + i].x);
-  for (int e = threadIdx.x; e < N * N; e += CHOL_THREADS)
-    if (e / N <= e % N) g[e] = cm[e];
+  write_back();
 }
 
 // FP32 orbitals.  One cluster of CTAs per configuration (and group of 16 block

@@ -33,3 +33,21 @@ def test_minors(N, mode, which):
     got = torch.empty_like(want)
     ctx.check(lib().nrcps_slater_dets(ctx.handle, _ptr(s), _ptr(p), N, 5, mode, 0, _ptr(got)))
     assert ((got - want).abs() <= 1e-11 * want.abs()).all()
+
+
+@pytest.mark.parametrize("N", [1, 5, 19, 33, 64])
+@pytest.mark.parametrize("dtype", [torch.complex64, torch.complex128])
+def test_reorthonormalise_scratch(N, dtype):
+    """The caller's scratch on 8 bytes: the same bits as on 16."""
+    import nrcps_b200 as nb
+    from nrcps_b200.api import lib, _ptr
+    ctx = nb.default_context()
+    g = torch.Generator(device=ctx.device).manual_seed(N)
+    psi = torch.randn((3, N, 512), dtype=dtype, device=ctx.device, generator=g)
+    want, logR = psi.clone(), torch.zeros((3, N), dtype=torch.float64, device=ctx.device)
+    nb.reorthonormalise(want, logR, ctx)
+    got, log8 = psi.clone(), torch.zeros_like(logR)
+    work = _on_eight(torch.zeros((3, N, N), dtype=torch.complex128, device=ctx.device))
+    ctx.check(lib().nrcps_reorthonormalise(ctx.handle, _ptr(got), N, 512, 3, 0 if dtype == torch.complex128 else 1,
+                                           _ptr(work), _ptr(log8)))
+    assert torch.equal(got, want) and torch.equal(log8, logR)
