@@ -94,6 +94,7 @@ extern "C" nrcps_status nrcps_destroy(nrcps_context* ctx) {
   for (void* u : ctx->unit)
     if (u) cudaFree(u);
   if (ctx->overlap_part) cudaFree(ctx->overlap_part);
+  if (ctx->overlap_done) cudaEventDestroy(ctx->overlap_done);
   if (ctx->dev_err) cudaFree(ctx->dev_err);
   delete ctx;
   return NRCPS_OK;

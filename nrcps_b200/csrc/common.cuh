@@ -114,6 +114,7 @@ struct Context {
   size_t tc_split_bytes = 0;
   void* unit[64] = {};  // tables of ones for a fused step without k(p) or field, by lattice extent
   void* overlap_part = nullptr;  // chunk sums of the CUDA-core overlap (fixed size, made at the first use)
+  cudaEvent_t overlap_done = nullptr;  // the last use of overlap_part, waited for by the next
   int* dev_err = nullptr;
   int* dev_pair_flag = nullptr;  // the word after dev_err: 1 = the last checked opposite-site table is no involution  // device flag set by kernels whose bounded waits time out
   // Time limit of every mbarrier wait in the fused step (nanoseconds of the

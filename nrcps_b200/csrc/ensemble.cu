@@ -21,8 +21,8 @@ nrcps_status slater_dets_dispatch(nrcps_context* ctx, const double* S, const dou
                               int log_det, double* out, long out_conf_stride, long out_offset, double* scr);
 size_t slater_dets_scratch_bytes(int N, int nconf, int mode);
 nrcps_status overlap_impl(nrcps_context* ctx, const double* src, int ns, const void* psi, int nt, int nconf,
-                          long vol, nrcps_precision prec, double* S);
-nrcps_status overlap_reserve(nrcps_context* ctx);
+                          long vol, nrcps_precision prec, double* S, double* part);
+size_t overlap_part_bytes(nrcps_context* ctx, int ns, int nt, int nconf, long vol);
 nrcps_status gather_impl(nrcps_context* ctx, const int* index, int ns, const void* psi, int nt, int nconf, long vol,
                          nrcps_precision prec, double* S);
 nrcps_status pair_impl(nrcps_context* ctx, const void* psi1, const void* psi2, int n, int nconf, long vol,
@@ -45,6 +45,7 @@ struct nrcps_ensemble {
   size_t esize = 0;  // bytes per complex orbital entry
   void* psi = nullptr;
   double* src = nullptr;
+  double* src_part = nullptr;  // chunk sums of the CUDA-core overlap, where a second kernel adds them up
   float* src_split = nullptr;  // TF32 hi/lo sources of the tensor-core overlap (FP32 orbitals)
   int* pw_index = nullptr;
   double* kinv = nullptr;
@@ -156,7 +157,7 @@ static nrcps_status record_time_loop(nrcps_ensemble* e, double* dets) {
     if (j.mode == 0) {
       if (e->pw_index) NRCPS_TRY(gather_impl(ctx, e->pw_index, N, e->psi, N, nc, vol, prec, e->S));
       else if (e->src_split) NRCPS_TRY(overlap_tc(ctx, e->src_split, N, e->psi, N, nc, vol, e->S));
-      else NRCPS_TRY(overlap_impl(ctx, e->src, N, e->psi, N, nc, vol, prec, e->S));
+      else NRCPS_TRY(overlap_impl(ctx, e->src, N, e->psi, N, nc, vol, prec, e->S, e->src_part));
       NRCPS_TRY(slater_dets_dispatch(ctx, e->S, nullptr, N, nc, 0, 0, dets, 2L * T * e->nmeas, 2L * t * e->nmeas,
                                  e->lu_scr));
       if (e->qr_logR && t >= j.qr_period)
@@ -165,7 +166,7 @@ static nrcps_status record_time_loop(nrcps_ensemble* e, double* dets) {
       NRCPS_TRY(pair_impl(ctx, e->psi, e->psi, N, nc, vol, e->w, e->opp, prec, e->S, e->pair_props));
       if (e->pw_index) NRCPS_TRY(gather_impl(ctx, e->pw_index, N, e->psi, N, nc, vol, prec, e->P1));
       else if (e->src_split) NRCPS_TRY(overlap_tc(ctx, e->src_split, N, e->psi, N, nc, vol, e->P1));
-      else NRCPS_TRY(overlap_impl(ctx, e->src, N, e->psi, N, nc, vol, prec, e->P1));
+      else NRCPS_TRY(overlap_impl(ctx, e->src, N, e->psi, N, nc, vol, prec, e->P1, e->src_part));
       NRCPS_TRY(slater_dets_dispatch(ctx, e->S, e->P1, N, nc, 1, 0, dets, 2L * T * e->nmeas, 2L * t * e->nmeas,
                                  e->lu_scr));
       if (e->qr_logR && t >= j.qr_period)
@@ -279,7 +280,7 @@ extern "C" nrcps_status nrcps_ensemble_create(nrcps_context* ctx, const nrcps_jo
       if ((st = dalloc(ctx, (char**)&e->src_split, overlap_tc_split_bytes(N, V))) ||
           (st = overlap_tc_prepare(ctx, e->src, N, V, N, nc, e->src_split)))
         return fail(st);
-    } else if ((st = overlap_reserve(ctx))) {  // the time loop is captured: nothing is allocated there
+    } else if ((st = dalloc(ctx, (char**)&e->src_part, overlap_part_bytes(ctx, N, N, nc, V)))) {
       return fail(st);
     }
   }
@@ -421,7 +422,7 @@ extern "C" nrcps_status nrcps_ensemble_destroy(nrcps_ensemble* e) {
   if (e->exec) cudaGraphExecDestroy(e->exec);
   if (e->graph) cudaGraphDestroy(e->graph);
   void* bufs[] = {e->psi, e->src, e->src_split, e->pw_index, e->kinv, e->kinv_f, e->pos, e->zpos, e->itab, e->w, e->opp,
-                  e->bits, e->phi, e->fld, e->S, e->P1, e->lu_scr, e->qr_G, e->qr_logR};
+                  e->src_part, e->bits, e->phi, e->fld, e->S, e->P1, e->lu_scr, e->qr_G, e->qr_logR};
   for (void* b : bufs)
     if (b) cudaFree(b);
   delete e;

@@ -1124,41 +1124,67 @@ nrcps_status slater_dets_dispatch(nrcps_context* ctx, const double* S, const dou
   return slater_dets_impl(ctx, S, psi1, N, nconf, mode, log_det, out, out_conf_stride, out_offset, scr);
 }
 
-// The chunks' sums of overlap_tile_kernel: a buffer of fixed size, made at the
-// first use outside a stream capture.
+// The chunks' sums of overlap_tile_kernel, where a second kernel adds them up:
+// an ensemble, whose graph holds the address, brings a buffer of its own; a
+// direct call takes the context's, of fixed size and made at the first use,
+// after an event that the last call which used it recorded behind its second
+// kernel -- the context's stream may be another one by now.  A call inside a
+// capture takes neither: the graph may run beside later calls.
 constexpr size_t kOverlapPartBytes = 16u << 20;
-nrcps_status overlap_reserve(nrcps_context* ctx) {
-  if (ctx->overlap_part) return NRCPS_OK;
-  return check_cuda(ctx, cudaMalloc(&ctx->overlap_part, kOverlapPartBytes), "cudaMalloc(overlap sums)");
+
+static double* overlap_context_part(nrcps_context* ctx) {
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  cudaError_t e = cudaStreamIsCapturing(ctx->stream, &cs);
+  if (e == cudaSuccess && cs != cudaStreamCaptureStatusNone) return nullptr;
+  if (e == cudaSuccess && !ctx->overlap_done)
+    e = cudaEventCreateWithFlags(&ctx->overlap_done, cudaEventDisableTiming);
+  if (e == cudaSuccess && !ctx->overlap_part) e = cudaMalloc(&ctx->overlap_part, kOverlapPartBytes);
+  if (e == cudaSuccess) e = cudaStreamWaitEvent(ctx->stream, ctx->overlap_done, 0);
+  if (e == cudaSuccess) return (double*)ctx->overlap_part;
+  cudaGetLastError();
+  return nullptr;
+}
+
+// Chunks of a configuration's sites: about four CTAs per SM, at least eight
+// stages each, and what the buffer of their sums holds (more than eight leave
+// them there).
+static long overlap_chunks(const nrcps_context* ctx, const OvTile& o, int ns, int nt, int nconf, long vol) {
+  const long tiles = (long)nconf * o.ns_t * o.nt_t;
+  const size_t per_chunk = sizeof(double2) * (size_t)nconf * ns * nt;
+  long chunks = (4L * ctx->sm_count + tiles - 1) / tiles;
+  if (chunks > vol / (8L * o.T)) chunks = vol / (8L * o.T);
+  if (chunks > (long)(kOverlapPartBytes / per_chunk)) chunks = (long)(kOverlapPartBytes / per_chunk);
+  if (chunks > 8 && chunks <= 16) chunks = 8;  // (up to 16 the second kernel costs more than it gives)
+  return chunks < 1 ? 1 : chunks;
+}
+
+// What an ensemble of these overlaps brings for the sums (0: nothing).
+size_t overlap_part_bytes(nrcps_context* ctx, int ns, int nt, int nconf, long vol) {
+  const long chunks = overlap_chunks(ctx, overlap_tiles(ns, nt), ns, nt, nconf, vol);
+  return chunks > 8 ? sizeof(double2) * (size_t)nconf * ns * nt * chunks : 0;
 }
 
 template <typename R>
 static nrcps_status launch_overlap(nrcps_context* ctx, const double* src, int ns, const void* psi, int nt, int nconf,
-                                   long vol, double* S) {
+                                   long vol, double* S, double* part) {
   const OvTile o = overlap_tiles(ns, nt);
   const size_t smem = sizeof(double2) * 2 * (size_t)o.rows * o.T;
   NRCPS_TRY(check_cuda(ctx, cudaFuncSetAttribute(overlap_tile_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                  (int)smem),
                        "overlap_tile: smem attribute"));
-  // chunks: about four CTAs per SM, at least eight stages each, and what the buffer holds
   const int tiles = o.ns_t * o.nt_t;
-  const size_t per_chunk = sizeof(double2) * (size_t)nconf * ns * nt;
-  long chunks = (4L * ctx->sm_count + (long)nconf * tiles - 1) / ((long)nconf * tiles);
-  if (chunks > vol / (8L * o.T)) chunks = vol / (8L * o.T);
-  if (chunks > (long)(kOverlapPartBytes / per_chunk)) chunks = (long)(kOverlapPartBytes / per_chunk);
-  if (chunks > 8 && chunks <= 16) chunks = 8;  // (the second kernel costs more than it gives)
-  if (chunks > 8 && !ctx->overlap_part) {
-    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    cudaStreamIsCapturing(ctx->stream, &cs);
-    if (cs != cudaStreamCaptureStatusNone) chunks = 8;  // nothing is allocated inside a capture
-    else NRCPS_TRY(overlap_reserve(ctx));
+  long chunks = overlap_chunks(ctx, o, ns, nt, nconf, vol);
+  bool shared = false;
+  if (chunks > 8 && !part) {
+    part = overlap_context_part(ctx);
+    shared = part != nullptr;
+    if (!part) chunks = 8;
   }
-  if (chunks < 1) chunks = 1;
   const long sites = (vol + chunks - 1) / chunks;
   const long chunk_sites = (sites + o.T - 1) / o.T * o.T;
   chunks = (vol + chunk_sites - 1) / chunk_sites;
   const bool sums = chunks > 8;
-  double2* out = reinterpret_cast<double2*>(sums ? (double*)ctx->overlap_part : S);
+  double2* out = reinterpret_cast<double2*>(sums ? part : S);
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -1179,16 +1205,21 @@ static nrcps_status launch_overlap(nrcps_context* ctx, const double* src, int ns
     overlap_sum_kernel<<<grid_for(total, 64), 64, 0, ctx->stream>>>(out, (int)chunks, per_conf, total,
                                                                     reinterpret_cast<double2*>(S));
     ctx->launches++;
-    NRCPS_TRY(check_launch(ctx, "overlap_sum_kernel"));
+    const nrcps_status st = check_launch(ctx, "overlap_sum_kernel");
+    if (shared)
+      NRCPS_TRY(check_cuda(ctx, cudaEventRecord(ctx->overlap_done, ctx->stream), "overlap: event record"));
+    return st;
   }
   return NRCPS_OK;
 }
 
+// part: the caller's buffer of overlap_part_bytes() for the chunks' sums, or
+// null for the context's.
 nrcps_status overlap_impl(nrcps_context* ctx, const double* src, int ns, const void* psi, int nt, int nconf,
-                          long vol, nrcps_precision prec, double* S) {
+                          long vol, nrcps_precision prec, double* S, double* part) {
   if ((long)nconf * nt * ns == 0) return NRCPS_OK;
-  return prec == NRCPS_F64 ? launch_overlap<double>(ctx, src, ns, psi, nt, nconf, vol, S)
-                           : launch_overlap<float>(ctx, src, ns, psi, nt, nconf, vol, S);
+  return prec == NRCPS_F64 ? launch_overlap<double>(ctx, src, ns, psi, nt, nconf, vol, S, part)
+                           : launch_overlap<float>(ctx, src, ns, psi, nt, nconf, vol, S, part);
 }
 
 nrcps_status gather_impl(nrcps_context* ctx, const int* index, int ns, const void* psi, int nt, int nconf, long vol,
@@ -1306,7 +1337,7 @@ extern "C" nrcps_status nrcps_overlap(nrcps_context* ctx, const double* dev_src,
     NRCPS_TRY(overlap_tc_prepare(ctx, dev_src, ns, vol, nt, nconf, (float*)ctx->tc_split));
     return overlap_tc(ctx, (const float*)ctx->tc_split, ns, dev_psi, nt, nconf, vol, dev_S);
   }
-  return overlap_impl(ctx, dev_src, ns, dev_psi, nt, nconf, vol, prec, dev_S);
+  return overlap_impl(ctx, dev_src, ns, dev_psi, nt, nconf, vol, prec, dev_S, nullptr);
 }
 
 extern "C" nrcps_status nrcps_overlap_planewave(nrcps_context* ctx, const int* dev_index, int ns, const void* dev_psi,
