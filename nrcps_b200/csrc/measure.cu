@@ -10,20 +10,28 @@ namespace cg = cooperative_groups;
 
 // ---------------------------------------------------------------- overlap
 // S[c][s][t] = sum_p conj(src_s(p)) psi_{c,t}(p) in FP64 for both orbital
-// precisions.  A CTA takes a chunk of one configuration's sites and a tile of
-// up to 32 blocks of 4 sources x 4 orbitals; stages of T sites of all its
+// precisions.  A CTA takes consecutive chunks of one configuration's sites and a
+// tile of up to 32 blocks of 4 sources x 4 orbitals; stages of T sites of all its
 // rows pass through shared memory (cp.async, two buffers), thread (block, l)
 // sums its block over the sites l, l + lanes, ..: 8 sixteen-byte loads for 64
-// FP64 FMAs.  Up to eight chunks are a cluster, which sums them; of more, each
-// chunk's sums go to `out` by themselves and overlap_sum_kernel adds them up.
-// Both in chunk order.
+// FP64 FMAs.
+//
+// The order of every sum is given by (ns, nt, vol) alone, so that a
+// configuration's overlap has the same bits in every batch, on every stream and
+// in a graph: a chunk by the lanes, then their tree; the chunks of a group (an
+// eighth) one after the other; the groups one after the other.  Who does which
+// is free: one CTA all of a configuration, a cluster a group per CTA, or, where
+// few configurations leave the chip idle, a CTA a few chunks whose sums go to
+// `out` one by one and overlap_sum_kernel adds up.
 //
 // Why chunks: one configuration's overlap is 47 M FP64 FMAs at N = 19, L = 32,
 // 3 us of the whole chip, and the reference's drivers measure one
-// configuration at a time.  Measured (FP64, call by call): that one 40 us, most
-// of it launch and latency (a block per orbital: 226); 64 configurations 0.54
-// ms against 1.64, 3.0 G FMAs at 30 % of the FP64 pipe, where the shared-memory
-// loads (45 %), the barriers of a stage and the FMAs take turns.
+// configuration at a time.  Measured (FP64, call by call): that one 34 us, most
+// of it launch and latency (a block per orbital: 216); 40 configurations 0.47
+// ms against 1.06, 300 2.53 against 6.89, 30 % of the FP64 pipe, where the
+// shared-memory loads (45 %), the barriers of a stage and the FMAs take turns.
+// A chunk's tree costs a tenth there (sums that followed the batch: 0.41 and
+// 2.59).
 constexpr int OV_THREADS = 256;
 
 struct OvTile {
@@ -50,27 +58,52 @@ __host__ __device__ inline OvTile overlap_tiles(int ns, int nt) {
   return o;
 }
 
+// Chunks of a configuration's sites and their groups.  At least 512 sites and 32
+// per lane: a chunk's tree and its share of the sums cost about a tenth of its
+// FMAs there; at most 512 chunks (the sums' buffer).
+constexpr int OV_GROUPS = 8;
+struct OvChunks {
+  long sites;                       // of a chunk, a multiple of T
+  int chunks, per_group, groups;
+};
+__host__ __device__ inline OvChunks overlap_chunks(const OvTile& o, long vol) {
+  OvChunks c;
+  c.sites = 32L * o.lanes < 512 ? 512 : 32L * o.lanes;
+  while ((vol + c.sites - 1) / c.sites > 512) c.sites *= 2;
+  c.chunks = (int)((vol + c.sites - 1) / c.sites);
+  c.per_group = (c.chunks + OV_GROUPS - 1) / OV_GROUPS;
+  c.groups = (c.chunks + c.per_group - 1) / c.per_group;
+  return c;
+}
+
+// CTA r of the `ctas` of a configuration and tile takes chunks r per_cta .. ;
+// each: every chunk's sums to out[conf][chunk], else out[conf] the whole sum (one
+// CTA, or a cluster of one per group).
 template <typename R>
-__global__ void __launch_bounds__(OV_THREADS) overlap_tile_kernel(const double2* __restrict__ src, int ns,
-                                                                  const void* __restrict__ psi, int nt, long vol,
-                                                                  int chunks, long chunk_sites, OvTile o,
-                                                                  double2* __restrict__ out) {
-  extern __shared__ __align__(16) double2 ovs[];  // [2][rows][T]
+__global__ void __launch_bounds__(OV_THREADS, 2) overlap_tile_kernel(const double2* __restrict__ src, int ns,
+                                                                  const void* __restrict__ psi, int nt, int nconf,
+                                                                  long vol, int ctas, int per_cta, int each,
+                                                                  OvChunks ch, OvTile o, double* __restrict__ out) {
+  extern __shared__ __align__(16) double2 ovs[];  // [2][rows][T], then [2][16 blocks]
   const int T = o.T, lanes = o.lanes;
-  const long conf = blockIdx.x / chunks;
-  const int chunk = (int)(blockIdx.x - conf * chunks);
-  const int s0 = 4 * o.ts * (int)(blockIdx.y % o.ns_t), t0 = 4 * o.tt * (int)(blockIdx.y / o.ns_t);
-  const long p0 = chunk * chunk_sites, p1 = p0 + chunk_sites < vol ? p0 + chunk_sites : vol;
+  const long task = blockIdx.x / ctas;
+  const int r = (int)(blockIdx.x - task * ctas);
+  const long conf = task % nconf;
+  const int tile = (int)(task / nconf);
+  const int s0 = 4 * o.ts * (tile % o.ns_t), t0 = 4 * o.tt * (tile / o.ns_t);
+  int chunk = r * per_cta;
+  const int last = chunk + per_cta < ch.chunks ? chunk + per_cta : ch.chunks;
+  const long p0 = chunk * ch.sites, p1 = last * ch.sites < vol ? last * ch.sites : vol;
   const cplx<R>* orb = reinterpret_cast<const cplx<R>*>(psi) + (size_t)conf * nt * vol;
   const int l = threadIdx.x % lanes, slot = threadIdx.x / lanes;
   const bool active = slot < o.ts * o.tt;
   const int bi = active ? slot / o.tt : 0, bj = active ? slot % o.tt : 0;
   auto fill = [&](long p, double2* t) {
     for (int e = threadIdx.x; e < o.rows * T; e += OV_THREADS) {
-      const int r = e >> o.log_t;
+      const int row = e >> o.log_t;
       const long q = p + (e & (T - 1));
-      const bool is_src = r < 4 * o.ts;
-      const int i = is_src ? s0 + r : t0 + r - 4 * o.ts;
+      const bool is_src = row < 4 * o.ts;
+      const int i = is_src ? s0 + row : t0 + row - 4 * o.ts;
       if (q >= p1 || i >= (is_src ? ns : nt)) {
         t[e] = make_double2(0.0, 0.0);
       } else if (is_src || sizeof(R) == 8) {
@@ -84,10 +117,30 @@ __global__ void __launch_bounds__(OV_THREADS) overlap_tile_kernel(const double2*
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
+  const int size = o.rows * T;
+  // the sums of this thread's block: all groups', and the present one's.  A lane
+  // ends a chunk with entries `mine` .. (two of 8 lanes, one of 16; of 32 every
+  // other lane one)
+  double2* all = ovs + 2 * size + 16 * slot;
+  double2* group = all + 16 * o.ts * o.tt;
+  const int held = lanes == 8 ? 2 : 1;
+  const bool owner = active && (lanes < 32 || l % 2 == 0);
+  int mine = 0;
+#pragma unroll
+  for (int h = 8; h >= 1; h >>= 1)
+    if (l & (lanes * h / 16)) mine += h;
+  if (owner)
+    for (int j = 0; j < held; ++j) all[mine + j] = group[mine + j] = make_double2(0.0, 0.0);
   double re[16], im[16];
 #pragma unroll
   for (int k = 0; k < 16; ++k) re[k] = im[k] = 0.0;
-  const int size = o.rows * T;
+  auto store = [&](size_t matrix, int k, double2 v) {
+    const int s = s0 + 4 * bi + k / 4, t = t0 + 4 * bj + k % 4;
+    if (s >= ns || t >= nt) return;
+    double* to = out + 2 * ((matrix * ns + s) * nt + t);  // (the caller's S: on 8 bytes)
+    to[0] = v.x;
+    to[1] = v.y;
+  };
   fill(p0, ovs);
   int buf = 0;
   for (long p = p0; p < p1; p += T, buf ^= 1) {
@@ -119,66 +172,105 @@ __global__ void __launch_bounds__(OV_THREADS) overlap_tile_kernel(const double2*
         }
       }
     }
-  }
-  // the lanes of a block are neighbours in one warp
-  for (int off = lanes / 2; off > 0; off >>= 1)
+    if (p + T < p1 && p + T < (chunk + 1) * ch.sites) continue;
+    // the chunk is done: the tree over a block's lanes, neighbours in one warp,
+    // which halve the entries between them at each level
 #pragma unroll
-    for (int k = 0; k < 16; ++k) {
-      re[k] += __shfl_xor_sync(0xffffffffu, re[k], off);
-      im[k] += __shfl_xor_sync(0xffffffffu, im[k], off);
-    }
-  cg::cluster_group cluster = cg::this_cluster();
-  const int split = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
-  if (split == 1) {
-    if (active && l == 0)
+    for (int h = 8; h >= 1; h >>= 1) {
+      const int off = lanes * h / 16;
+      if (off == 0) continue;
+      const bool up = l & off;
 #pragma unroll
-      for (int k = 0; k < 16; ++k) {
-        const int s = s0 + 4 * bi + k / 4, t = t0 + 4 * bj + k % 4;
-        if (s < ns && t < nt) out[((size_t)blockIdx.x * ns + s) * nt + t] = make_double2(re[k], im[k]);
+      for (int k = 0; k < h; ++k) {
+        const double kr = up ? re[k + h] : re[k], sr = up ? re[k] : re[k + h];
+        const double ki = up ? im[k + h] : im[k], si = up ? im[k] : im[k + h];
+        re[k] = kr + __shfl_xor_sync(0xffffffffu, sr, off);
+        im[k] = ki + __shfl_xor_sync(0xffffffffu, si, off);
       }
+    }
+    if (lanes == 32) {
+      re[0] += __shfl_xor_sync(0xffffffffu, re[0], 1);
+      im[0] += __shfl_xor_sync(0xffffffffu, im[0], 1);
+    }
+    const bool closes = (chunk + 1) % ch.per_group == 0 || chunk + 1 == ch.chunks;
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      if (!owner || j >= held) continue;
+      const double2 v = make_double2(re[j], im[j]);
+      if (each) {
+        store((size_t)conf * ch.chunks + chunk, mine + j, v);
+      } else {
+        double2 g = group[mine + j];
+        g.x += v.x;
+        g.y += v.y;
+        if (closes) {
+          all[mine + j].x += g.x;
+          all[mine + j].y += g.y;
+          g = make_double2(0.0, 0.0);
+        }
+        group[mine + j] = g;
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < 16; ++k) re[k] = im[k] = 0.0;
+    ++chunk;
+  }
+  if (each) return;
+  if (ctas == 1) {
+    if (owner)
+      for (int j = 0; j < held; ++j) store(conf, mine + j, all[mine + j]);
     return;
   }
-  // a cluster holds all chunks of its configuration: entries spread over its CTAs
-  __syncthreads();
-  if (active && l == 0)
-#pragma unroll
-    for (int k = 0; k < 16; ++k) ovs[16 * slot + k] = make_double2(re[k], im[k]);
+  // a cluster holds the groups of its configuration: entries spread over its CTAs
+  cg::cluster_group cluster = cg::this_cluster();
   cluster.sync();
-  for (int e = rank * OV_THREADS + threadIdx.x; e < 16 * o.ts * o.tt; e += split * OV_THREADS) {
+  for (int e = r * OV_THREADS + threadIdx.x; e < 16 * o.ts * o.tt; e += ctas * OV_THREADS) {
     double2 v = make_double2(0.0, 0.0);
-    for (int r = 0; r < split; ++r) {
-      const double2 w = cluster.map_shared_rank(ovs, r)[e];
+    for (int g = 0; g < ctas; ++g) {
+      const double2 w = cluster.map_shared_rank(ovs + 2 * size, g)[e];
       v.x += w.x;
       v.y += w.y;
     }
     const int b = e / 16, s = s0 + 4 * (b / o.tt) + e % 16 / 4, t = t0 + 4 * (b % o.tt) + e % 4;
-    if (s < ns && t < nt) out[((size_t)conf * ns + s) * nt + t] = v;
+    if (s < ns && t < nt) {
+      double* to = out + 2 * (((size_t)conf * ns + s) * nt + t);
+      to[0] = v.x;
+      to[1] = v.y;
+    }
   }
   cluster.sync();  // peers keep their shared memory until every sum is read
 }
 
-// S[c][e] = sum over the chunks, in order; sixteen loads in flight (one by one
+// S[c][e] = the chunks' sums, group by group; sixteen loads in flight (one by one
 // the 64 chunks of a single configuration, N = 19, L = 32, took 19.5 us; now
 // 10.0).
-__global__ void overlap_sum_kernel(const double2* __restrict__ part, int chunks, long per_conf, long total,
-                                   double2* __restrict__ S) {
+__global__ void overlap_sum_kernel(const double2* __restrict__ part, OvChunks ch, long per_conf, long total,
+                                   double* __restrict__ S) {
   for (long e = (long)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (long)gridDim.x * blockDim.x) {
     const long c = e / per_conf, i = e - c * per_conf;
-    const double2* p = part + (size_t)c * chunks * per_conf + i;
-    double2 v = make_double2(0.0, 0.0);
-    for (int k0 = 0; k0 < chunks; k0 += 16) {
+    const double2* p = part + (size_t)c * ch.chunks * per_conf + i;
+    double2 v = make_double2(0.0, 0.0), group = v;
+    int left = ch.per_group;  // chunks to come of the present group
+    for (int k0 = 0; k0 < ch.chunks; k0 += 16) {
       double2 w[16];
 #pragma unroll
       for (int k = 0; k < 16; ++k)
-        if (k0 + k < chunks) w[k] = __ldcg(p + (size_t)(k0 + k) * per_conf);
+        if (k0 + k < ch.chunks) w[k] = __ldcg(p + (size_t)(k0 + k) * per_conf);
 #pragma unroll
       for (int k = 0; k < 16; ++k)
-        if (k0 + k < chunks) {
-          v.x += w[k].x;
-          v.y += w[k].y;
+        if (k0 + k < ch.chunks) {
+          group.x += w[k].x;
+          group.y += w[k].y;
+          if (--left == 0 || k0 + k + 1 == ch.chunks) {
+            v.x += group.x;
+            v.y += group.y;
+            group = make_double2(0.0, 0.0);
+            left = ch.per_group;
+          }
         }
     }
-    S[e] = v;
+    S[2 * e] = v.x;
+    S[2 * e + 1] = v.y;
   }
 }
 
@@ -1130,7 +1222,7 @@ nrcps_status slater_dets_dispatch(nrcps_context* ctx, const double* S, const dou
 // after an event that the last call which used it recorded behind its second
 // kernel -- the context's stream may be another one by now.  A call inside a
 // capture takes neither: the graph may run beside later calls.
-constexpr size_t kOverlapPartBytes = 16u << 20;
+constexpr size_t kOverlapPartBytes = 32u << 20;  // (N = 19 at L = 48: 26 configurations)
 
 static double* overlap_context_part(nrcps_context* ctx) {
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
@@ -1145,52 +1237,50 @@ static double* overlap_context_part(nrcps_context* ctx) {
   return nullptr;
 }
 
-// Chunks of a configuration's sites: about four CTAs per SM, at least eight
-// stages each, and what the buffer of their sums holds (more than eight leave
-// them there).
-static long overlap_chunks(const nrcps_context* ctx, const OvTile& o, int ns, int nt, int nconf, long vol) {
+// CTAs for a configuration and tile: about four per SM in all.  One takes it
+// alone, a cluster has one per group; more than twice the groups (below, the
+// second kernel costs more than it gives) leave their chunks' sums in a buffer.
+static long overlap_ctas(const nrcps_context* ctx, const OvTile& o, const OvChunks& ch, int ns, int nt, int nconf) {
   const long tiles = (long)nconf * o.ns_t * o.nt_t;
-  const size_t per_chunk = sizeof(double2) * (size_t)nconf * ns * nt;
-  long chunks = (4L * ctx->sm_count + tiles - 1) / tiles;
-  if (chunks > vol / (8L * o.T)) chunks = vol / (8L * o.T);
-  if (chunks > (long)(kOverlapPartBytes / per_chunk)) chunks = (long)(kOverlapPartBytes / per_chunk);
-  if (chunks > 8 && chunks <= 16) chunks = 8;  // (up to 16 the second kernel costs more than it gives)
-  return chunks < 1 ? 1 : chunks;
+  const long want = (4L * ctx->sm_count + tiles - 1) / tiles;
+  if (want <= 1 || ch.groups == 1) return 1;
+  const bool room = sizeof(double2) * (size_t)nconf * ns * nt * ch.chunks <= kOverlapPartBytes;
+  if (want <= 2 * OV_GROUPS || ch.chunks <= 2 * OV_GROUPS || !room) return ch.groups;
+  const long per = (ch.chunks + want - 1) / want;
+  return (ch.chunks + per - 1) / per;
 }
 
 // What an ensemble of these overlaps brings for the sums (0: nothing).
 size_t overlap_part_bytes(nrcps_context* ctx, int ns, int nt, int nconf, long vol) {
-  const long chunks = overlap_chunks(ctx, overlap_tiles(ns, nt), ns, nt, nconf, vol);
-  return chunks > 8 ? sizeof(double2) * (size_t)nconf * ns * nt * chunks : 0;
+  const OvTile o = overlap_tiles(ns, nt);
+  const OvChunks ch = overlap_chunks(o, vol);
+  return overlap_ctas(ctx, o, ch, ns, nt, nconf) > ch.groups ? sizeof(double2) * (size_t)nconf * ns * nt * ch.chunks : 0;
 }
 
 template <typename R>
 static nrcps_status launch_overlap(nrcps_context* ctx, const double* src, int ns, const void* psi, int nt, int nconf,
                                    long vol, double* S, double* part) {
   const OvTile o = overlap_tiles(ns, nt);
-  const size_t smem = sizeof(double2) * 2 * (size_t)o.rows * o.T;
+  const OvChunks ch = overlap_chunks(o, vol);
+  const size_t smem = sizeof(double2) * (2 * (size_t)o.rows * o.T + 2 * 16 * o.ts * o.tt);
   NRCPS_TRY(check_cuda(ctx, cudaFuncSetAttribute(overlap_tile_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                  (int)smem),
                        "overlap_tile: smem attribute"));
-  const int tiles = o.ns_t * o.nt_t;
-  long chunks = overlap_chunks(ctx, o, ns, nt, nconf, vol);
+  long ctas = overlap_ctas(ctx, o, ch, ns, nt, nconf);
   bool shared = false;
-  if (chunks > 8 && !part) {
+  if (ctas > ch.groups && !part) {
     part = overlap_context_part(ctx);
     shared = part != nullptr;
-    if (!part) chunks = 8;
+    if (!part) ctas = ch.groups;
   }
-  const long sites = (vol + chunks - 1) / chunks;
-  const long chunk_sites = (sites + o.T - 1) / o.T * o.T;
-  chunks = (vol + chunk_sites - 1) / chunk_sites;
-  const bool sums = chunks > 8;
-  double2* out = reinterpret_cast<double2*>(sums ? part : S);
+  const bool each = ctas > ch.groups;
+  const int per_cta = each ? (int)((ch.chunks + ctas - 1) / ctas) : ctas == 1 ? ch.chunks : ch.per_group;
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = sums ? 1u : (unsigned)chunks;
+  attr[0].val.clusterDim.x = each ? 1u : (unsigned)ctas;
   attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-  cfg.gridDim = dim3((unsigned)(nconf * chunks), (unsigned)tiles);
+  cfg.gridDim = dim3((unsigned)((long)nconf * o.ns_t * o.nt_t * ctas));
   cfg.blockDim = dim3(OV_THREADS);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = ctx->stream;
@@ -1198,12 +1288,13 @@ static nrcps_status launch_overlap(nrcps_context* ctx, const double* src, int ns
   cfg.numAttrs = 1;
   ctx->launches++;
   NRCPS_TRY(check_cuda(ctx, cudaLaunchKernelEx(&cfg, overlap_tile_kernel<R>, reinterpret_cast<const double2*>(src), ns,
-                                               psi, nt, vol, (int)chunks, chunk_sites, o, out),
+                                               psi, nt, nconf, vol, (int)ctas, per_cta, each ? 1 : 0, ch, o,
+                                               each ? part : S),
                        "overlap_tile_kernel launch"));
-  if (sums) {
+  if (each) {
     const long per_conf = (long)ns * nt, total = nconf * per_conf;
-    overlap_sum_kernel<<<grid_for(total, 64), 64, 0, ctx->stream>>>(out, (int)chunks, per_conf, total,
-                                                                    reinterpret_cast<double2*>(S));
+    overlap_sum_kernel<<<grid_for(total, 64), 64, 0, ctx->stream>>>(reinterpret_cast<const double2*>(part), ch,
+                                                                    per_conf, total, S);
     ctx->launches++;
     const nrcps_status st = check_launch(ctx, "overlap_sum_kernel");
     if (shared)

@@ -1,0 +1,37 @@
+"""The CUDA-core overlap's order of summation: given by the shape, not by the
+batch, the buffer at hand or a capture."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("ns,nt,vol", [(19, 19, 13824), (7, 7, 4096), (3, 2, 5000), (33, 20, 1000), (16, 40, 4096),
+                                       (5, 9, 700)])
+@pytest.mark.parametrize("precision", ["f64", "f32"])
+def test_same_bits_in_every_batch(ns, nt, vol, precision):
+    """One configuration alone (many CTAs), in batches that give it a cluster
+    or one CTA, and in a graph: the same bits."""
+    import nrcps_b200 as nb
+    ctx = nb.Context(0)
+    g = torch.Generator(device=ctx.device).manual_seed(ns * 100 + nt)
+    dt = torch.complex128 if precision == "f64" else torch.complex64
+    src = torch.randn((ns, vol), dtype=torch.complex128, device=ctx.device, generator=g)
+    batch = [1, 2, 40, 100, 700] if vol * nt < 1 << 17 else [1, 2, 30, 90]
+    psi = torch.randn((max(batch), nt, vol), dtype=dt, device=ctx.device, generator=g)
+    ctx.set_option("overlap.tc", 0)
+    want = nb.overlap(src, psi[:1], ctx)
+    for n in batch:
+        got = nb.overlap(src, psi[:n], ctx)
+        assert torch.equal(got[:1], want), n
+        assert torch.equal(got[n - 1:], nb.overlap(src, psi[n - 1:n], ctx)), n
+    s, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph, stream=s):
+        ctx.use_current_stream()
+        out = nb.overlap(src, psi[:1], ctx)
+    ctx.use_current_stream()
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(out, want)
+    ctx.close()
