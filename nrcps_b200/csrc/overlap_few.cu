@@ -209,7 +209,7 @@ nrcps_status launch_few(nrcps_context* ctx, const float* src, int ns, const void
 // 5, 800 310 against 401; but L = 48, n = 7, 180 591 against 488, n = 1, 500 496
 // against 174, L = 16, n = 10, 4000 670 against 531.
 bool overlap_few_pays(int ns, int nt, int nconf, long vol) {
-  if (ns > 2 * FB) return false;
+  if (ns > 2 * FB || nt > 65535L * 2 * FB) return false;  // (groups of orbitals are a grid's y)
   if ((double)nconf * nt * vol <= (double)(1 << 24)) return true;
   const int padded = (ns + FB - 1) / FB * ((nt + FB - 1) / FB) * FB * FB;
   return 4 * padded <= 5 * ns * nt && vol >= 32 * 32 * 32;

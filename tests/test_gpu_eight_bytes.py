@@ -51,3 +51,20 @@ def test_reorthonormalise_scratch(N, dtype):
     ctx.check(lib().nrcps_reorthonormalise(ctx.handle, _ptr(got), N, 512, 3, 0 if dtype == torch.complex128 else 1,
                                            _ptr(work), _ptr(log8)))
     assert torch.equal(got, want) and torch.equal(log8, logR)
+
+
+@pytest.mark.parametrize("nconf", [1, 6, 200])
+def test_overlap_into_eight_bytes(nconf):
+    """S on 8 bytes from one CTA, a cluster and many CTAs per configuration:
+    the same bits as on 16."""
+    import nrcps_b200 as nb
+    from nrcps_b200.api import lib, _ptr
+    ctx = nb.default_context()
+    ns, nt, vol = 19, 18, 13824
+    g = torch.Generator(device=ctx.device).manual_seed(nconf)
+    src = torch.randn((ns, vol), dtype=torch.complex128, device=ctx.device, generator=g)
+    psi = torch.randn((nconf, nt, vol), dtype=torch.complex128, device=ctx.device, generator=g)
+    want = torch.view_as_real(nb.overlap(src, psi, ctx)).reshape(-1)
+    out = _on_eight(torch.zeros((nconf, ns, nt), dtype=torch.complex128, device=ctx.device))
+    ctx.check(lib().nrcps_overlap(ctx.handle, _ptr(src), ns, _ptr(psi), nt, nconf, vol, 0, _ptr(out)))
+    assert torch.equal(out[:want.numel()], want)

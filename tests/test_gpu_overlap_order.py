@@ -35,3 +35,20 @@ def test_same_bits_in_every_batch(ns, nt, vol, precision):
     torch.cuda.synchronize()
     assert torch.equal(out, want)
     ctx.close()
+
+
+@pytest.mark.parametrize("precision,nt,vol", [("f64", 1600000, 4), ("f32", 700000, 16)])
+def test_very_many_orbitals(precision, nt, vol):
+    """More tiles and groups of orbitals than a grid has in y: accepted as by a
+    block per orbital.  Sums of at most 16 products, in FP32 or better."""
+    import nrcps_b200 as nb
+    ctx = nb.default_context()
+    g = torch.Generator(device=ctx.device).manual_seed(nt)
+    dt = torch.complex128 if precision == "f64" else torch.complex64
+    src = torch.randn((1, vol), dtype=torch.complex128, device=ctx.device, generator=g)
+    psi = torch.randn((1, nt, vol), dtype=dt, device=ctx.device, generator=g)
+    got = nb.overlap(src, psi, ctx)
+    p = psi.to(torch.complex128)
+    want = torch.einsum("sv,ctv->cst", src.conj(), p)
+    size = torch.einsum("sv,ctv->cst", src.abs(), p.abs())
+    assert ((got - want).abs() <= (1e-14 if precision == "f64" else 3e-6) * size).all()
