@@ -27,11 +27,9 @@ namespace cg = cooperative_groups;
 // Why chunks: one configuration's overlap is 47 M FP64 FMAs at N = 19, L = 32,
 // 3 us of the whole chip, and the reference's drivers measure one
 // configuration at a time.  Measured (FP64, call by call): that one 34 us, most
-// of it launch and latency (a block per orbital: 216); 40 configurations 0.47
-// ms against 1.06, 300 2.53 against 6.89, 30 % of the FP64 pipe, where the
+// of it launch and latency (a block per orbital: 216); 40 configurations 0.36
+// ms against 1.06, 300 2.51 against 6.89, 30 % of the FP64 pipe, where the
 // shared-memory loads (45 %), the barriers of a stage and the FMAs take turns.
-// A chunk's tree costs a tenth there (sums that followed the batch: 0.41 and
-// 2.59).
 constexpr int OV_THREADS = 256;
 
 struct OvTile {
@@ -51,29 +49,64 @@ __host__ __device__ inline OvTile overlap_tiles(int ns, int nt) {
   }
   o.ns_t = (bs + o.ts - 1) / o.ts, o.nt_t = (bt + o.tt - 1) / o.tt;
   o.rows = 4 * (o.ts + o.tt);
-  o.log_t = o.rows <= 8 ? 7 : o.rows <= 48 ? 6 : 5;  // both buffers of two CTAs fit an SM up to 48 rows
+  // both buffers of two CTAs fit an SM up to 48 rows
+  o.log_t = o.rows <= 8 ? 8 : o.rows <= 24 ? 7 : o.rows <= 48 ? 6 : 5;
   o.T = 1 << o.log_t;
   o.lanes = 8;
   while (2 * o.lanes * o.ts * o.tt <= OV_THREADS && 2 * o.lanes <= 32) o.lanes *= 2;
   return o;
 }
 
-// Chunks of a configuration's sites and their groups.  At least 512 sites and 32
-// per lane: a chunk's tree and its share of the sums cost about a tenth of its
-// FMAs there; at most 512 chunks (the sums' buffer).
+// Chunks of a configuration's sites and their groups.  512 sites: a chunk's tree
+// and its share of the sums cost about a tenth of its FMAs there; half as many in
+// small volumes, where a call waits for its longest CTA (N = 19, L = 8: 17 us, one
+// chunk of 512 25); at most 512 chunks (the sums' buffer).
 constexpr int OV_GROUPS = 8;
 struct OvChunks {
   long sites;                       // of a chunk, a multiple of T
   int chunks, per_group, groups;
 };
-__host__ __device__ inline OvChunks overlap_chunks(const OvTile& o, long vol) {
+__host__ __device__ inline OvChunks overlap_chunks(long vol) {
   OvChunks c;
-  c.sites = 32L * o.lanes < 512 ? 512 : 32L * o.lanes;
+  c.sites = vol <= 2048 ? 256 : 512;
   while ((vol + c.sites - 1) / c.sites > 512) c.sites *= 2;
   c.chunks = (int)((vol + c.sites - 1) / c.sites);
   c.per_group = (c.chunks + OV_GROUPS - 1) / OV_GROUPS;
   c.groups = (c.chunks + c.per_group - 1) / c.per_group;
   return c;
+}
+
+// The end of a chunk: the tree over an entry's lanes, neighbours in one warp, which
+// halve the N entries between them at each level while there are any to halve.
+// Lane l is left with the sums of the entries from overlap_first<N>(l, lanes) on.
+template <int N>
+__device__ __forceinline__ void overlap_tree(double (&re)[N], double (&im)[N], int l, int lanes) {
+  int off = lanes / 2;
+#pragma unroll
+  for (int h = N / 2; h >= 1; h >>= 1) {
+    if (off == 0) continue;
+    const bool up = l & off;
+#pragma unroll
+    for (int k = 0; k < h; ++k) {
+      const double kr = up ? re[k + h] : re[k], sr = up ? re[k] : re[k + h];
+      const double ki = up ? im[k + h] : im[k], si = up ? im[k] : im[k + h];
+      re[k] = kr + __shfl_xor_sync(0xffffffffu, sr, off);
+      im[k] = ki + __shfl_xor_sync(0xffffffffu, si, off);
+    }
+    off >>= 1;
+  }
+  for (; off > 0; off >>= 1) {
+    re[0] += __shfl_xor_sync(0xffffffffu, re[0], off);
+    im[0] += __shfl_xor_sync(0xffffffffu, im[0], off);
+  }
+}
+template <int N>
+__device__ __forceinline__ int overlap_first(int l, int lanes) {
+  int e = 0, off = lanes / 2;
+#pragma unroll
+  for (int h = N / 2; h >= 1; h >>= 1, off >>= 1)
+    if (l & off) e += h;
+  return e;
 }
 
 // CTA r of the `ctas` of a configuration and tile takes chunks r per_cta .. ;
@@ -110,25 +143,33 @@ __global__ void __launch_bounds__(OV_THREADS, 2) overlap_tile_kernel(const doubl
         const void* g = is_src ? (const void*)(src + (size_t)i * vol + q) : (const void*)(orb + (size_t)i * vol + q);
         asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(t + e)), "l"(g)
                      : "memory");
-      } else {
-        const cplx<R> v = orb[(size_t)i * vol + q];
-        t[e] = make_double2((double)v.re, (double)v.im);
+      } else {  // FP32: into the element's upper half, spread by `widen`
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((uint32_t)__cvta_generic_to_shared(&t[e].y)),
+                     "l"(orb + (size_t)i * vol + q)
+                     : "memory");
       }
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
+  // FP32 orbitals to FP64 in place, by the thread that copied them
+  const int first = (int)threadIdx.x + 4 * o.ts * T / OV_THREADS * OV_THREADS;
+  auto widen = [&](long p, double2* t) {
+    for (int e = first; e < o.rows * T; e += OV_THREADS) {
+      const int row = e >> o.log_t;
+      const long q = p + (e & (T - 1));
+      if (row >= 4 * o.ts && q < p1 && t0 + row - 4 * o.ts < nt) {
+        const float2 v = *reinterpret_cast<const float2*>(&t[e].y);
+        t[e] = make_double2((double)v.x, (double)v.y);
+      }
+    }
+  };
   const int size = o.rows * T;
-  // the sums of this thread's block: all groups', and the present one's.  A lane
-  // ends a chunk with entries `mine` .. (two of 8 lanes, one of 16; of 32 every
-  // other lane one)
+  // the sums of this thread's block: all groups', and the present one's
   double2* all = ovs + 2 * size + 16 * slot;
   double2* group = all + 16 * o.ts * o.tt;
   const int held = lanes == 8 ? 2 : 1;
   const bool owner = active && (lanes < 32 || l % 2 == 0);
-  int mine = 0;
-#pragma unroll
-  for (int h = 8; h >= 1; h >>= 1)
-    if (l & (lanes * h / 16)) mine += h;
+  const int mine = overlap_first<16>(l, lanes);
   if (owner)
     for (int j = 0; j < held; ++j) all[mine + j] = group[mine + j] = make_double2(0.0, 0.0);
   double re[16], im[16];
@@ -148,6 +189,7 @@ __global__ void __launch_bounds__(OV_THREADS, 2) overlap_tile_kernel(const doubl
     if (p + T < p1) fill(p + T, ovs + (buf ^ 1) * size);
     else asm volatile("cp.async.commit_group;" ::: "memory");
     asm volatile("cp.async.wait_group 1;" ::: "memory");
+    if (sizeof(R) == 4) widen(p, ovs + buf * size);
     __syncthreads();
     if (active) {
       const double2* ta = ovs + buf * size + 4 * bi * T;
@@ -173,25 +215,7 @@ __global__ void __launch_bounds__(OV_THREADS, 2) overlap_tile_kernel(const doubl
       }
     }
     if (p + T < p1 && p + T < (chunk + 1) * ch.sites) continue;
-    // the chunk is done: the tree over a block's lanes, neighbours in one warp,
-    // which halve the entries between them at each level
-#pragma unroll
-    for (int h = 8; h >= 1; h >>= 1) {
-      const int off = lanes * h / 16;
-      if (off == 0) continue;
-      const bool up = l & off;
-#pragma unroll
-      for (int k = 0; k < h; ++k) {
-        const double kr = up ? re[k + h] : re[k], sr = up ? re[k] : re[k + h];
-        const double ki = up ? im[k + h] : im[k], si = up ? im[k] : im[k + h];
-        re[k] = kr + __shfl_xor_sync(0xffffffffu, sr, off);
-        im[k] = ki + __shfl_xor_sync(0xffffffffu, si, off);
-      }
-    }
-    if (lanes == 32) {
-      re[0] += __shfl_xor_sync(0xffffffffu, re[0], 1);
-      im[0] += __shfl_xor_sync(0xffffffffu, im[0], 1);
-    }
+    overlap_tree(re, im, l, lanes);
     const bool closes = (chunk + 1) % ch.per_group == 0 || chunk + 1 == ch.chunks;
 #pragma unroll
     for (int j = 0; j < 2; ++j) {
@@ -239,6 +263,67 @@ __global__ void __launch_bounds__(OV_THREADS, 2) overlap_tile_kernel(const doubl
     }
   }
   cluster.sync();  // peers keep their shared memory until every sum is read
+}
+
+// The same sums for up to eight sources where an entry has 32 lanes, without
+// staging: a warp takes one orbital and one group of its chunks, SB sources in
+// registers; the groups of an orbital meet in shared memory.  With few sources
+// there is little to reuse, the orbitals are the traffic, and the tile kernel
+// keeps too few bytes in flight (a 4 x 4 block mostly padding on top): N = 2, FP64,
+// 1000 configurations at L = 48 688 us (5.1 TB/s) against 4.2 ms, 300 at L = 32
+// 85 against 407; a block per orbital: 1328 and 163.
+constexpr int OD_WARPS = 8;
+template <typename R, int SB>
+__global__ void __launch_bounds__(32 * OD_WARPS, SB == 8 ? 2 : 3)
+    overlap_direct_kernel(const double2* __restrict__ src, int ns, const void* __restrict__ psi, int nt, long vol,
+                          long orbitals, OvChunks ch, double* __restrict__ S) {
+  __shared__ double2 sums[OD_WARPS][SB];
+  const int l = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int here = OD_WARPS / ch.groups, g = warp % ch.groups;  // orbitals of this CTA, the warp's group
+  const long first = (long)blockIdx.x * here, orbital = first + warp / ch.groups;
+  const bool active = warp < here * ch.groups && orbital < orbitals;
+  const cplx<R>* orb = reinterpret_cast<const cplx<R>*>(psi) + (size_t)(active ? orbital : 0) * vol;
+  double gr = 0.0, gi = 0.0;
+  const int last = !active ? 0 : (g + 1) * ch.per_group < ch.chunks ? (g + 1) * ch.per_group : ch.chunks;
+  for (int chunk = g * ch.per_group; chunk < last; ++chunk) {
+    double re[SB], im[SB];
+#pragma unroll
+    for (int k = 0; k < SB; ++k) re[k] = im[k] = 0.0;
+    const long end = (chunk + 1) * ch.sites < vol ? (chunk + 1) * ch.sites : vol;
+#pragma unroll 4
+    for (long q = chunk * ch.sites + l; q < end; q += 32) {
+      const cplx<R> v = orb[q];
+      const double br = (double)v.re, bi = (double)v.im;
+      double2 a[SB];
+#pragma unroll
+      for (int u = 0; u < SB; ++u) a[u] = u < ns ? __ldg(src + (size_t)u * vol + q) : make_double2(0.0, 0.0);
+#pragma unroll
+      for (int u = 0; u < SB; ++u) {
+        re[u] = fma(a[u].x, br, re[u]);
+        im[u] = fma(a[u].x, bi, im[u]);
+        re[u] = fma(a[u].y, bi, re[u]);
+        im[u] = fma(-a[u].y, br, im[u]);
+      }
+    }
+    overlap_tree<SB>(re, im, l, 32);
+    gr += re[0];
+    gi += im[0];
+  }
+  if (l % (32 / SB) == 0) sums[warp][overlap_first<SB>(l, 32)] = make_double2(gr, gi);
+  __syncthreads();
+  for (int e = threadIdx.x; e < here * SB; e += 32 * OD_WARPS) {
+    const int s = e % SB, k = e / SB;
+    if (s >= ns || first + k >= orbitals) continue;
+    double2 v = make_double2(0.0, 0.0);
+    for (int i = 0; i < ch.groups; ++i) {
+      v.x += sums[k * ch.groups + i][s].x;
+      v.y += sums[k * ch.groups + i][s].y;
+    }
+    const long conf = (first + k) / nt, t = (first + k) % nt;
+    double* to = S + 2 * ((conf * ns + s) * nt + t);
+    to[0] = v.x;
+    to[1] = v.y;
+  }
 }
 
 // S[c][e] = the chunks' sums, group by group; sixteen loads in flight (one by one
@@ -1238,49 +1323,79 @@ static double* overlap_context_part(nrcps_context* ctx) {
 }
 
 // CTAs for a configuration and tile: about four per SM in all.  One takes it
-// alone, a cluster has one per group; more than twice the groups (below, the
-// second kernel costs more than it gives) leave their chunks' sums in a buffer.
-static long overlap_ctas(const nrcps_context* ctx, const OvTile& o, const OvChunks& ch, int ns, int nt, int nconf) {
+// alone, a cluster has one per group; where more than four are wanted they leave
+// their chunks' sums in a buffer for a second kernel (`each`): clusters of seven
+// or eight do not fill the chip.  FP64, 40 configurations of N = 19, L = 32: 355 us
+// against 455 by clusters, L = 24 148 against 221; 100 of them 355 and 419.
+struct OvSplit {
+  int ctas, per_cta;
+  bool each;
+};
+static OvSplit overlap_split(const nrcps_context* ctx, const OvTile& o, const OvChunks& ch, int ns, int nt, int nconf,
+                             bool buffer) {
   const long tiles = (long)nconf * o.ns_t * o.nt_t;
   const long want = (4L * ctx->sm_count + tiles - 1) / tiles;
-  if (want <= 1 || ch.groups == 1) return 1;
+  if (want <= 1 || ch.groups == 1) return {1, ch.chunks, false};
   const bool room = sizeof(double2) * (size_t)nconf * ns * nt * ch.chunks <= kOverlapPartBytes;
-  if (want <= 2 * OV_GROUPS || ch.chunks <= 2 * OV_GROUPS || !room) return ch.groups;
+  if (want <= 4 || ch.chunks <= OV_GROUPS || !room || !buffer)
+    return {ch.groups, ch.per_group, false};
   const long per = (ch.chunks + want - 1) / want;
-  return (ch.chunks + per - 1) / per;
+  return {(int)((ch.chunks + per - 1) / per), (int)per, true};
+}
+
+// Where the kernel without staging is the faster one: a chunk per group at most
+// (up to L = 16), or orbitals enough to fill the chip.  It against the tile kernel,
+// FP64, us: N = 7, L = 16, 40 configurations 16 / 22; N = 7, L = 32, 4
+// configurations 40 / 23, 16 42 / 48; N = 4, L = 32, one 33 / 17, 40 70 / 89; N = 8,
+// L = 16, 300 93 / 106, 1000 282 / 256.
+static bool overlap_direct_pays(int ns, int nt, int nconf, bool fp64, const OvTile& o, const OvChunks& ch) {
+  if (o.lanes < 32 || ns > 8) return false;
+  const long orbitals = (long)nconf * nt;
+  if (fp64 && ns > 4 && orbitals > 4096) return false;
+  return ch.per_group == 1 || orbitals >= 10L * ns;
 }
 
 // What an ensemble of these overlaps brings for the sums (0: nothing).
 size_t overlap_part_bytes(nrcps_context* ctx, int ns, int nt, int nconf, long vol) {
   const OvTile o = overlap_tiles(ns, nt);
-  const OvChunks ch = overlap_chunks(o, vol);
-  return overlap_ctas(ctx, o, ch, ns, nt, nconf) > ch.groups ? sizeof(double2) * (size_t)nconf * ns * nt * ch.chunks : 0;
+  const OvChunks ch = overlap_chunks(vol);
+  return overlap_split(ctx, o, ch, ns, nt, nconf, true).each ? sizeof(double2) * (size_t)nconf * ns * nt * ch.chunks : 0;
 }
 
 template <typename R>
 static nrcps_status launch_overlap(nrcps_context* ctx, const double* src, int ns, const void* psi, int nt, int nconf,
                                    long vol, double* S, double* part) {
   const OvTile o = overlap_tiles(ns, nt);
-  const OvChunks ch = overlap_chunks(o, vol);
+  const OvChunks ch = overlap_chunks(vol);
+  if (overlap_direct_pays(ns, nt, nconf, sizeof(R) == 8, o, ch)) {
+    const long orbitals = (long)nconf * nt, here = OD_WARPS / ch.groups;
+    auto launch = [&](auto kern) {
+      kern<<<(unsigned)((orbitals + here - 1) / here), 32 * OD_WARPS, 0, ctx->stream>>>(
+          reinterpret_cast<const double2*>(src), ns, psi, nt, vol, orbitals, ch, S);
+    };
+    if (ns <= 2) launch(overlap_direct_kernel<R, 2>);
+    else if (ns <= 4) launch(overlap_direct_kernel<R, 4>);
+    else launch(overlap_direct_kernel<R, 8>);
+    ctx->launches++;
+    return check_launch(ctx, "overlap_direct_kernel");
+  }
   const size_t smem = sizeof(double2) * (2 * (size_t)o.rows * o.T + 2 * 16 * o.ts * o.tt);
   NRCPS_TRY(check_cuda(ctx, cudaFuncSetAttribute(overlap_tile_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                  (int)smem),
                        "overlap_tile: smem attribute"));
-  long ctas = overlap_ctas(ctx, o, ch, ns, nt, nconf);
+  OvSplit split = overlap_split(ctx, o, ch, ns, nt, nconf, true);
   bool shared = false;
-  if (ctas > ch.groups && !part) {
+  if (split.each && !part) {
     part = overlap_context_part(ctx);
     shared = part != nullptr;
-    if (!part) ctas = ch.groups;
+    if (!part) split = overlap_split(ctx, o, ch, ns, nt, nconf, false);
   }
-  const bool each = ctas > ch.groups;
-  const int per_cta = each ? (int)((ch.chunks + ctas - 1) / ctas) : ctas == 1 ? ch.chunks : ch.per_group;
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = each ? 1u : (unsigned)ctas;
+  attr[0].val.clusterDim.x = split.each ? 1u : (unsigned)split.ctas;
   attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-  cfg.gridDim = dim3((unsigned)((long)nconf * o.ns_t * o.nt_t * ctas));
+  cfg.gridDim = dim3((unsigned)((long)nconf * o.ns_t * o.nt_t * split.ctas));
   cfg.blockDim = dim3(OV_THREADS);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = ctx->stream;
@@ -1288,10 +1403,10 @@ static nrcps_status launch_overlap(nrcps_context* ctx, const double* src, int ns
   cfg.numAttrs = 1;
   ctx->launches++;
   NRCPS_TRY(check_cuda(ctx, cudaLaunchKernelEx(&cfg, overlap_tile_kernel<R>, reinterpret_cast<const double2*>(src), ns,
-                                               psi, nt, nconf, vol, (int)ctas, per_cta, each ? 1 : 0, ch, o,
-                                               each ? part : S),
+                                               psi, nt, nconf, vol, split.ctas, split.per_cta, split.each ? 1 : 0, ch,
+                                               o, split.each ? part : S),
                        "overlap_tile_kernel launch"));
-  if (each) {
+  if (split.each) {
     const long per_conf = (long)ns * nt, total = nconf * per_conf;
     overlap_sum_kernel<<<grid_for(total, 64), 64, 0, ctx->stream>>>(reinterpret_cast<const double2*>(part), ch,
                                                                     per_conf, total, S);

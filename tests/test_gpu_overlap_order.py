@@ -7,7 +7,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("ns,nt,vol", [(19, 19, 13824), (7, 7, 4096), (3, 2, 5000), (33, 20, 1000), (16, 40, 4096),
-                                       (5, 9, 700)])
+                                       (5, 9, 700), (7, 7, 13824), (2, 2, 13824), (4, 5, 2048), (10, 10, 1728)])
 @pytest.mark.parametrize("precision", ["f64", "f32"])
 def test_same_bits_in_every_batch(ns, nt, vol, precision):
     """One configuration alone (many CTAs), in batches that give it a cluster
