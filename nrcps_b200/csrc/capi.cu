@@ -28,6 +28,13 @@ nrcps_status check_launch(nrcps_context* ctx, const char* what) {
   return check_cuda(ctx, cudaGetLastError(), what);
 }
 
+nrcps_status allow_smem(nrcps_context* ctx, const void* kern, size_t most, const char* what) {
+  if (ctx->kernels.count(kern)) return NRCPS_OK;
+  NRCPS_TRY(check_cuda(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most), what));
+  ctx->kernels[kern] = 0;
+  return NRCPS_OK;
+}
+
 void* scratch(nrcps_context* ctx, size_t bytes, nrcps_status* st) {
   *st = NRCPS_OK;
   // a side-stream field draw may still be using the scratch (no scratch

@@ -6,6 +6,7 @@
 
 #include <cstdio>
 #include <string>
+#include <unordered_map>
 
 #include "../../include/nrcps_b200.h"
 
@@ -113,6 +114,9 @@ struct Context {
   void* tc_split = nullptr;
   size_t tc_split_bytes = 0;
   void* unit[64] = {};  // tables of ones for a fused step without k(p) or field, by lattice extent
+  // Kernels whose attributes this context has set, and for the clustered ones
+  // how many clusters fit the device (allow_smem, launch_fused).
+  std::unordered_map<const void*, int> kernels;
   void* overlap_part = nullptr;  // chunk sums of the CUDA-core overlap (fixed size, made at the first use)
   cudaEvent_t overlap_done = nullptr;  // the last use of overlap_part, waited for by the next
   int* dev_err = nullptr;
@@ -141,6 +145,11 @@ nrcps_status set_error(nrcps_context* ctx, nrcps_status st, const char* fmt, ...
 nrcps_status check_cuda(nrcps_context* ctx, cudaError_t e, const char* what);
 nrcps_status check_launch(nrcps_context* ctx, const char* what);
 void* scratch(nrcps_context* ctx, size_t bytes, nrcps_status* st);
+
+// Lets `kern` have up to `most` bytes of dynamic shared memory; asked of the driver
+// once per context.  The limit is the device's, whatever context or thread set it
+// last, so `most` is what any launch of the kernel may need, never one call's size.
+nrcps_status allow_smem(nrcps_context* ctx, const void* kern, size_t most, const char* what);
 
 inline long vol_of(const int dims[3]) { return (long)dims[0] * dims[1] * dims[2]; }
 

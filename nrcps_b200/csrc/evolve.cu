@@ -104,6 +104,7 @@ __global__ void __launch_bounds__(256) evolve_kernel(const cplx<R>* in, cplx<R>*
   }
 }
 
+constexpr size_t kEvolveSmem = 227 * 1024;
 size_t evolve_smem(size_t esz, const int d[3]) { return esz * (size_t)d[0] * d[1] * (d[2] + 1); }
 
 template <typename R, int SIGN, int OP, bool INIT>
@@ -111,8 +112,7 @@ nrcps_status launch_evolve(nrcps_context* ctx, const void* in, void* out, int ba
                            const double* table) {
   const size_t smem = evolve_smem(sizeof(cplx<R>), d);
   auto kern = evolve_kernel<R, SIGN, OP, INIT>;
-  NRCPS_TRY(check_cuda(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
-                       "evolve: smem attribute"));
+  NRCPS_TRY(allow_smem(ctx, (const void*)kern, kEvolveSmem, "evolve: smem attribute"));
   // a thread per pencil of the axis with the most, at most 256
   int most = d[0] * d[1] > d[0] * d[2] ? d[0] * d[1] : d[0] * d[2];
   if (d[1] * d[2] > most) most = d[1] * d[2];
@@ -127,7 +127,7 @@ nrcps_status launch_evolve(nrcps_context* ctx, const void* in, void* out, int ba
 
 // Whether one orbital of these extents fits a CTA's shared memory.
 bool evolve_fits(nrcps_precision prec, const int d[3]) {
-  return evolve_smem(prec == NRCPS_F64 ? sizeof(cplx<double>) : sizeof(cplx<float>), d) <= 227 * 1024;
+  return evolve_smem(prec == NRCPS_F64 ? sizeof(cplx<double>) : sizeof(cplx<float>), d) <= kEvolveSmem;
 }
 
 // psi <- B[w . F[psi]] with w complex (interleaved FP64) or real (FP64).

@@ -21,8 +21,6 @@
 // fastest variant at that size), 2100 orbitals 42 against 49.  At L = 24 an
 // FP64 orbital fills the SM, its loads meet no other work, and the cluster of
 // four is faster (627 orbitals, Gaussian: 166 against 150 us).
-#include <atomic>
-
 #include "fused.cuh"
 
 namespace nrcps {
@@ -159,13 +157,7 @@ nrcps_status launch_one(nrcps_context* ctx, const FusedArgs& f) {
   using Sh = OneShape<R>;
   const bool z2 = f.field_mode == 1 && (f.pos == nullptr || f.zpos != nullptr);
   void (*kern)(FusedArgs) = z2 ? fused_step_one_kernel<R, 1> : fused_step_one_kernel<R, 2>;
-  static std::atomic<bool> ready[2][16];  // the attribute, once per kernel and device
-  std::atomic<bool>* known = ctx->device >= 0 && ctx->device < 16 ? &ready[z2][ctx->device] : nullptr;
-  if (!known || !known->load(std::memory_order_acquire)) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Sh::SMEM);
-    if (e != cudaSuccess) return check_cuda(ctx, e, "fused_step_one: smem attribute");
-    if (known) known->store(true, std::memory_order_release);
-  }
+  NRCPS_TRY(allow_smem(ctx, (const void*)kern, Sh::SMEM, "fused_step_one: smem attribute"));
   const long slots = (long)ctx->sm_count * Sh::CTAS;
   const long grid = f.n_orb_total < slots ? f.n_orb_total : slots;
   kern<<<(unsigned)grid, Sh::THREADS, Sh::SMEM, ctx->stream>>>(f);

@@ -43,8 +43,6 @@
 // The transforms are those of the cluster kernels operation by operation
 // (fft::Dft<32>: its even and odd halves meet only in the last radix-4
 // stage), so the results are the same bit for bit.
-#include <atomic>
-
 #include "fused.cuh"
 
 namespace nrcps {
@@ -411,15 +409,7 @@ nrcps_status fused_park_step(nrcps_context* ctx, const FusedArgs& f) {
   void (*kern)(FusedArgs) = z2                  ? fused_step_park_kernel<1>
                             : f.field_mode == 3 ? fused_step_park_kernel<3>
                                                 : fused_step_park_kernel<2>;
-  // (once per kernel and device: a call into the driver on every step otherwise)
-  static std::atomic<bool> ready[3][16];
-  std::atomic<bool>* known = ctx->device >= 0 && ctx->device < 16 ? &ready[z2 ? 0 : f.field_mode == 3 ? 2 : 1][ctx->device]
-                                                                  : nullptr;
-  if (!known || !known->load(std::memory_order_acquire)) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PSMEM);
-    if (e != cudaSuccess) return check_cuda(ctx, e, "fused_step_park: smem attribute");
-    if (known) known->store(true, std::memory_order_release);
-  }
+  NRCPS_TRY(allow_smem(ctx, (const void*)kern, PSMEM, "fused_step_park: smem attribute"));
   const long grid = f.n_orb_total < ctx->sm_count ? f.n_orb_total : ctx->sm_count;
   kern<<<(unsigned)grid, PTHREADS, PSMEM, ctx->stream>>>(f);
   ctx->launches++;

@@ -26,8 +26,6 @@
 // (plus the L2-resident k table and field bits).
 #include <cooperative_groups.h>
 
-#include <atomic>
-
 #include "fused.cuh"
 
 namespace cg = cooperative_groups;
@@ -1297,7 +1295,6 @@ static nrcps_status launch_fused(nrcps_context* ctx, const FusedArgs& f, int cta
                           : (KIND == 7 || KIND == 8) ? PullShape<R, L, C, false>::SMEM
                                                      : Sh::SMEM;
   void (*kern)(FusedArgs);
-  int inst = 0;  // which of the kind's kernels
   if constexpr (KIND == 1) kern = fused_step_split_kernel<R, L, C>;
   else if constexpr (KIND == 2) kern = fused_step_bulk_kernel<R, L, C, true>;
   else if constexpr (KIND == 3) kern = fused_step_bulk_kernel<R, L, C, false>;
@@ -1313,15 +1310,11 @@ static nrcps_status launch_fused(nrcps_context* ctx, const FusedArgs& f, int cta
     // position factor) or any other field
     const bool z2 = f.field_mode == 1 && (L * L) % 32 == 0 && (f.pos == nullptr || f.zpos != nullptr);
     kern = z2 ? fused_step_async_kernel<R, L, C, KIND == 12, 1> : fused_step_async_kernel<R, L, C, KIND == 12, 2>;
-    if (!z2) {
-      SMEM = AsyncShape<R, L, C, 2>::SMEM;
-      inst = 1;
-    }
+    if (!z2) SMEM = AsyncShape<R, L, C, 2>::SMEM;
     if constexpr (sizeof(R) == 4) {
       if (f.field_mode == 3) {  // (FP32 only: the host sends mode 3 with FP32 orbitals alone)
         kern = fused_step_async_kernel<R, L, C, KIND == 12, 3>;
         SMEM = AsyncShape<R, L, C, 3>::SMEM;
-        inst = 2;
       }
     }
   }
@@ -1339,15 +1332,13 @@ static nrcps_status launch_fused(nrcps_context* ctx, const FusedArgs& f, int cta
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   cfg.gridDim = dim3(C * ctx->sm_count);
-  // the attributes and the clusters that fit are asked for once per kernel
-  // (an instance per field class) and device: 3 us of the host on every step
-  static std::atomic<int> fit[3][16];
-  std::atomic<int>* known = ctx->device >= 0 && ctx->device < 16 ? &fit[inst][ctx->device] : nullptr;
-  int max_clusters = known ? known->load(std::memory_order_acquire) : 0;
-  cudaError_t e = cudaSuccess;
+  // the attributes and the clusters that fit are asked for once per kernel and
+  // context: 3 us of the host on every step
+  NRCPS_TRY(allow_smem(ctx, (const void*)kern, SMEM, "fused_step: smem attribute"));
+  int& known = ctx->kernels[(const void*)kern];
+  int max_clusters = known;
   if (max_clusters == 0) {
-    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM);
-    if (e != cudaSuccess) return check_cuda(ctx, e, "fused_step: smem attribute");
+    cudaError_t e = cudaSuccess;
     if (C > 8) {
       e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
       if (e != cudaSuccess) return check_cuda(ctx, e, "fused_step: cluster attribute");
@@ -1357,8 +1348,8 @@ static nrcps_status launch_fused(nrcps_context* ctx, const FusedArgs& f, int cta
       cudaGetLastError();
       max_clusters = ctx->sm_count / C;
       if (max_clusters < 1) return set_error(ctx, NRCPS_ERR_UNSUPPORTED, "fused_step: cluster of %d does not fit", C);
-    } else if (known) {
-      known->store(max_clusters, std::memory_order_release);
+    } else {
+      known = max_clusters;
     }
   }
   (void)ctas_per_sm_hint;
@@ -1366,7 +1357,7 @@ static nrcps_status launch_fused(nrcps_context* ctx, const FusedArgs& f, int cta
   if (clusters > f.n_orb_total) clusters = f.n_orb_total;
   if (clusters < 1) clusters = 1;
   cfg.gridDim = dim3((unsigned)(clusters * C));
-  e = cudaLaunchKernelEx(&cfg, kern, f);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, f);
   ctx->launches++;
   return check_cuda(ctx, e, "fused_step_kernel launch");
 }

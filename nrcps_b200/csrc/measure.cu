@@ -1380,9 +1380,8 @@ static nrcps_status launch_overlap(nrcps_context* ctx, const double* src, int ns
     return check_launch(ctx, "overlap_direct_kernel");
   }
   const size_t smem = sizeof(double2) * (2 * (size_t)o.rows * o.T + 2 * 16 * o.ts * o.tt);
-  NRCPS_TRY(check_cuda(ctx, cudaFuncSetAttribute(overlap_tile_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                 (int)smem),
-                       "overlap_tile: smem attribute"));
+  // (132 rows of 32 sites and 32 blocks are the most)
+  NRCPS_TRY(allow_smem(ctx, (const void*)overlap_tile_kernel<R>, 160 * 1024, "overlap_tile: smem attribute"));
   OvSplit split = overlap_split(ctx, o, ch, ns, nt, nconf, true);
   bool shared = false;
   if (split.each && !part) {

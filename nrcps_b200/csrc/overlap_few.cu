@@ -172,8 +172,7 @@ nrcps_status launch_few(nrcps_context* ctx, const float* src, int ns, const void
                         double* S) {
   using Sh = FewShape<NS, NT>;
   auto kern = overlap_few_kernel<NS, NT>;
-  NRCPS_TRY(check_cuda(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Sh::SMEM),
-                       "overlap_few: smem attribute"));
+  NRCPS_TRY(allow_smem(ctx, (const void*)kern, Sh::SMEM, "overlap_few: smem attribute"));
   // the split of a configuration that leaves the fewest rounds of CTAs per share
   const long groups = (nt + 2 * FB - 1) / (2 * FB), slots = (long)ctx->sm_count * FCTAS, ntiles = (vol + FT - 1) / FT;
   int split = 1;

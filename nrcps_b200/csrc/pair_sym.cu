@@ -312,8 +312,7 @@ nrcps_status launch_pair_sym(nrcps_context* ctx, const void* psi, int n, int nco
                              const int* opp, const int* flags, double* phi) {
   using Sh = SymShape<NB>;
   auto kern = pair_sym_kernel<NB>;
-  NRCPS_TRY(check_cuda(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Sh::SMEM),
-                       "pair_sym: smem attribute"));
+  NRCPS_TRY(allow_smem(ctx, (const void*)kern, Sh::SMEM, "pair_sym: smem attribute"));
   // the split of a configuration that leaves the fewest rounds of CTAs per share
   const long slots = (long)ctx->sm_count * Sh::CTAS, ntiles = (vol + ST - 1) / ST;
   int split = 1;

@@ -565,6 +565,8 @@ __global__ void rescale_dets_kernel(double* dets, const double* logR, int N, int
   }
 }
 
+constexpr size_t kMatrixSmem = sizeof(double2) * 64 * 64;  // N <= 64
+
 template <int NMAX>
 static nrcps_status launch_apply(nrcps_context* ctx, void* psi, int N, long vol, int nconf, nrcps_precision prec,
                                  const double* Rinv) {
@@ -581,8 +583,7 @@ static nrcps_status launch_apply(nrcps_context* ctx, void* psi, int N, long vol,
   if (sh > 48 * 1024) {
     const void* kern = prec == NRCPS_F64 ? (const void*)apply_rinv_kernel<double, NMAX>
                                          : (const void*)apply_rinv_kernel<float, NMAX>;
-    NRCPS_TRY(check_cuda(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh),
-                         "apply_rinv_kernel: smem attribute"));
+    NRCPS_TRY(allow_smem(ctx, kern, kMatrixSmem, "apply_rinv_kernel: smem attribute"));
   }
   if (prec == NRCPS_F64)
     apply_rinv_kernel<double, NMAX><<<(unsigned)(bpc * nconf), 256, sh, ctx->stream>>>(psi, N, vol, nconf, Rinv);
@@ -606,8 +607,7 @@ static nrcps_status launch_gram4(nrcps_context* ctx, const void* psi, int N, lon
     NRCPS_CASE(16)
 #undef NRCPS_CASE
   }
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh);
-  if (e != cudaSuccess) return check_cuda(ctx, e, "gram4: smem attribute");
+  NRCPS_TRY(allow_smem(ctx, (const void*)kern, sh, "gram4: smem attribute"));
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -658,7 +658,7 @@ nrcps_status qr_reorthonormalise(nrcps_context* ctx, void* psi, int N, long vol,
   }
   const size_t chol_sh = sizeof(double2) * N * N;
   if (chol_sh > 48 * 1024)
-    cudaFuncSetAttribute(chol_inv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)chol_sh);
+    NRCPS_TRY(allow_smem(ctx, (const void*)chol_inv_kernel, kMatrixSmem, "chol_inv_kernel: smem attribute"));
   chol_inv_kernel<<<(unsigned)nconf, CHOL_THREADS, chol_sh, ctx->stream>>>(G, N, logR, prec == NRCPS_F32);
   ctx->launches++;
   NRCPS_TRY(check_launch(ctx, "chol_inv_kernel"));
