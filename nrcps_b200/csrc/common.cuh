@@ -146,6 +146,20 @@ nrcps_status check_cuda(nrcps_context* ctx, cudaError_t e, const char* what);
 nrcps_status check_launch(nrcps_context* ctx, const char* what);
 void* scratch(nrcps_context* ctx, size_t bytes, nrcps_status* st);
 
+// While one lives, this thread's calls that make something at its first use
+// (cudaMalloc, cudaEventCreate, a wait) do not break the capture of another
+// thread's stream.
+class BesideCaptures {
+ public:
+  BesideCaptures() { cudaThreadExchangeStreamCaptureMode(&mode_); }
+  ~BesideCaptures() { cudaThreadExchangeStreamCaptureMode(&mode_); }
+  BesideCaptures(const BesideCaptures&) = delete;
+  BesideCaptures& operator=(const BesideCaptures&) = delete;
+
+ private:
+  cudaStreamCaptureMode mode_ = cudaStreamCaptureModeRelaxed;
+};
+
 // Lets `kern` have up to `most` bytes of dynamic shared memory; asked of the driver
 // once per context.  The limit is the device's, whatever context or thread set it
 // last, so `most` is what any launch of the kernel may need, never one call's size.

@@ -1313,6 +1313,7 @@ static double* overlap_context_part(nrcps_context* ctx) {
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
   cudaError_t e = cudaStreamIsCapturing(ctx->stream, &cs);
   if (e == cudaSuccess && cs != cudaStreamCaptureStatusNone) return nullptr;
+  BesideCaptures beside;
   if (e == cudaSuccess && !ctx->overlap_done)
     e = cudaEventCreateWithFlags(&ctx->overlap_done, cudaEventDisableTiming);
   if (e == cudaSuccess && !ctx->overlap_part) e = cudaMalloc(&ctx->overlap_part, kOverlapPartBytes);

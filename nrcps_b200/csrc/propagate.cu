@@ -281,6 +281,7 @@ static const double* unit_table(nrcps_context* ctx, int L) {
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
   cudaStreamIsCapturing(ctx->stream, &cs);
   if (cs != cudaStreamCaptureStatusNone) return nullptr;
+  BesideCaptures beside;
   const long V = (long)L * L * L;
   void* p = nullptr;
   if (cudaMalloc(&p, 32 * (size_t)V) != cudaSuccess) {

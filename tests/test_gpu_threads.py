@@ -56,3 +56,51 @@ def test_two_threads_with_kernels_of_different_sizes():
     assert not errors, errors
     for k in range(2):
         assert all(torch.equal(a, b) for a, b in zip(out[k], want[k]))
+
+
+def test_first_calls_beside_another_threads_capture():
+    """A first Evolve (a table of ones) and a first overlap of one configuration
+    (a buffer of sums) in one thread while another captures a graph: neither
+    call fails, nor does the capture."""
+    import nrcps_b200 as nb
+    from nrcps_b200.api import lib, _ip, _dims, _ptr
+    ctx = nb.Context(0)
+    L = 16
+    d3 = _ip(_dims((L, L, L)))
+    g = torch.Generator(device=ctx.device).manual_seed(5)
+    psi = torch.randn((2, L, L, L), dtype=torch.complex128, device=ctx.device, generator=g)
+    pot = torch.rand((L, L, L), dtype=torch.float64, device=ctx.device, generator=g) / L ** 3
+    src = torch.randn((19, 13824), dtype=torch.complex128, device=ctx.device, generator=g)
+    orb = torch.randn((1, 19, 13824), dtype=torch.complex128, device=ctx.device, generator=g)
+    S = torch.empty((1, 19, 19), dtype=torch.complex128, device=ctx.device)
+    x = torch.zeros(64, device=ctx.device)
+    side = torch.cuda.Stream()
+    with torch.cuda.stream(side):
+        ctx.use_current_stream()
+    other = nb.Context(0)
+    want = psi.clone()
+    other.check(lib().nrcps_potential_evolve(other.handle, _ptr(want), 2, d3, _ptr(pot), 0))
+    want_S = nb.overlap(src, orb, other)
+    torch.cuda.synchronize()
+    errors = []
+
+    def work():
+        try:
+            ctx.check(lib().nrcps_potential_evolve(ctx.handle, _ptr(psi), 2, d3, _ptr(pot), 0))
+            ctx.check(lib().nrcps_overlap(ctx.handle, _ptr(src), 19, _ptr(orb), 19, 1, 13824, 0, _ptr(S)))
+        except Exception as ex:  # noqa: BLE001
+            errors.append(ex)
+
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):  # (other threads' unsafe calls would end it)
+        x.add_(1.0)
+        t = threading.Thread(target=work)
+        t.start()
+        t.join()
+        x.mul_(2.0)
+    assert not errors, errors
+    graph.replay()
+    torch.cuda.synchronize()
+    assert x.eq(2.0).all() and torch.equal(psi, want) and torch.equal(S, want_S)
+    ctx.close()
+    other.close()
