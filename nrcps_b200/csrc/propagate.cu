@@ -23,7 +23,7 @@ struct PencilGeom {
   long stride;        // site stride along the pencil
 };
 
-enum PencilOp { OP_NONE = 0, OP_PRE_MUL = 1, OP_POST_MUL = 2, OP_MID_FIELD = 3, OP_MID_REAL = 4 };
+enum PencilOp { OP_NONE = 0, OP_PRE_MUL = 1, OP_POST_MUL = 2, OP_MID_FIELD = 3, OP_MID_REAL = 4, OP_MID_COMPLEX = 5 };
 
 struct FieldArgs {
   int mode;              // 0 complex fld, 1 Z2 bits, 2 interleaved complex phi, 3 real FP32 weights
@@ -92,6 +92,14 @@ __global__ void __launch_bounds__(128) pencil_kernel(void* data, long total, Pen
       const long conf = b / f.orbs_per_conf;
 #pragma unroll
       for (int j = 0; j < N; ++j) x[j] = cmul(field_factor<R>(f, w_plus, w_minus, conf, site0 + j * g.stride), x[j]);
+      fft::Dft<N, -SIGN, R>::run(x);
+    }
+    if constexpr (OP == OP_MID_COMPLEX) {  // (field_factor's branches would hold each site's load back)
+#pragma unroll
+      for (int j = 0; j < N; ++j) {
+        const double2 w = reinterpret_cast<const double2*>(table)[site0 + j * g.stride];
+        x[j] = cmul(cplx<R>{(R)w.x, (R)w.y}, x[j]);
+      }
       fft::Dft<N, -SIGN, R>::run(x);
     }
     if constexpr (OP == OP_MID_REAL) {
@@ -327,15 +335,12 @@ static nrcps_status evolve_any(nrcps_context* ctx, void* psi, int batch, const i
   // (a CTA per orbital: past some waves of them the pencil passes' better
   // occupancy wins, 2000 orbitals of 12^3 98 / 90 us)
   if (evolve_fits(prec, d) && batch <= 6 * ctx->sm_count) return evolve_step(ctx, psi, batch, d, w, w_complex, prec);
-  FieldArgs none{}, f{};
-  f.field = w;  // (mode 0)
-  f.vol = (double)vol_of(d);
-  f.orbs_per_conf = batch;
+  FieldArgs none{};
   auto passes = [&](auto zero) {
     using R = decltype(zero);
     NRCPS_TRY((launch_axis<R, -1, OP_NONE>(ctx, psi, batch, d, 2, nullptr, none)));
     NRCPS_TRY((launch_axis<R, -1, OP_NONE>(ctx, psi, batch, d, 1, nullptr, none)));
-    if (w_complex) NRCPS_TRY((launch_axis<R, -1, OP_MID_FIELD>(ctx, psi, batch, d, 0, nullptr, f)));
+    if (w_complex) NRCPS_TRY((launch_axis<R, -1, OP_MID_COMPLEX>(ctx, psi, batch, d, 0, w, none)));
     else NRCPS_TRY((launch_axis<R, -1, OP_MID_REAL>(ctx, psi, batch, d, 0, w, none)));
     NRCPS_TRY((launch_axis<R, +1, OP_NONE>(ctx, psi, batch, d, 1, nullptr, none)));
     return launch_axis<R, +1, OP_NONE>(ctx, psi, batch, d, 2, nullptr, none);
