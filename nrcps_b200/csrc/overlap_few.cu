@@ -200,18 +200,29 @@ nrcps_status launch_few(nrcps_context* ctx, const float* src, int ns, const void
 
 }  // namespace
 
-// Where this kernel is the faster one.  Small batches (128 MB of orbitals),
-// where the tensor-core kernel's preparation and fill show: L = 32, ten
-// orbitals, 30 configurations 53 against 94 us, 24 of seven at L = 8 23 against
-// 37.  Large ones where the blocks of five are nearly full and a configuration
-// has many tiles: L = 48, n = 10, 128 configurations 459 against 496, L = 32, n =
-// 5, 800 310 against 401; but L = 48, n = 7, 180 591 against 488, n = 1, 500 496
-// against 174, L = 16, n = 10, 4000 670 against 531.
+// Where this kernel is the faster one (measured with ns = nt = N).  Small batches
+// (128 MB of orbitals), where the tensor-core kernel's preparation and fill show:
+// L = 32, ten orbitals, 33 configurations 46 against 89 us, 24 of seven at L = 8
+// 15 against 22; but not those of very many configurations, which are a CTA each
+// at least (L = 8, N = 2, 1000 of them 32 against 21), nor of one to three sources
+// on many sites, where most of a block of five is padding (L = 48, N = 1, 100
+// configurations 98 against 61), nor, with more than five, large volumes, where
+// a cluster of eight per configuration leaves the chip empty (L = 48, N = 7, 16
+// configurations 122 against 73).  Large ones where the blocks of five are full
+// and a configuration has many tiles: L = 48, N = 10, 128 configurations 459
+// against 496 (16: 135 against 114), L = 32, N = 5, 1000 350 against 517; N = 9 up
+// to 128 configurations only (L = 32, 100 106 against 116, 500 486 against 442);
+// not L = 48, N = 7, 180: 591 against 488, nor L = 16, N = 10, 4000: 670 against 531.
 bool overlap_few_pays(int ns, int nt, int nconf, long vol) {
   if (ns > 2 * FB || nt > 65535L * 2 * FB) return false;  // (groups of orbitals are a grid's y)
-  if ((double)nconf * nt * vol <= (double)(1 << 24)) return true;
-  const int padded = (ns + FB - 1) / FB * ((nt + FB - 1) / FB) * FB * FB;
-  return 4 * padded <= 5 * ns * nt && vol >= 32 * 32 * 32;
+  const long l32 = 32 * 32 * 32, sites = nconf * vol;
+  if ((double)nt * sites <= (double)(1 << 24)) {
+    if (ns <= 3) return nconf <= 128 && sites <= 1 << 22;
+    return ns <= FB ? nconf <= 512 : nconf <= 320 && vol <= l32;
+  }
+  const long padded = (long)((ns + FB - 1) / FB) * ((nt + FB - 1) / FB) * FB * FB, full = (long)ns * nt;
+  return (9 * padded <= 10 * full || (4 * padded <= 5 * full && nconf <= 128)) && vol >= l32 &&
+         (ns <= FB || vol == l32 || nconf >= 32);
 }
 
 // The sources as FP32 in `out` (8 ns vol bytes, on 16).
