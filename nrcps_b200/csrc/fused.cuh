@@ -160,15 +160,22 @@ __device__ __forceinline__ cplx<R> scale_w(cplx<R> x, R hi, R lo);
 // x * w for a Z2 site with a position factor, from the table of both weights
 // of every site: the value apply_w_general gives (the table holds the same
 // products w_plus * P and w_minus * P, split the same way)
+template <typename R>
+struct ZposEntry {
+  typedef double2 type;
+};
+template <>
+struct ZposEntry<float> {
+  typedef float4 type;
+};
+template <typename R, bool PK>
+__device__ __forceinline__ cplx<R> scale_w_entry(typename ZposEntry<R>::type t, bool up, cplx<R> x) {
+  if constexpr (sizeof(R) == 4) return scale_w<R, PK>(x, up ? t.x : t.z, up ? t.y : t.w);
+  else return scale_w<R, PK>(x, up ? t.x : t.y, (R)0);
+}
 template <typename R, bool PK>
 __device__ __forceinline__ cplx<R> scale_w_zpos(const void* tab, int site, bool up, cplx<R> x) {
-  if constexpr (sizeof(R) == 4) {
-    const float4 t = __ldg(reinterpret_cast<const float4*>(tab) + site);
-    return scale_w<R, PK>(x, up ? t.x : t.z, up ? t.y : t.w);
-  } else {
-    const double2 t = __ldg(reinterpret_cast<const double2*>(tab) + site);
-    return scale_w<R, PK>(x, up ? t.x : t.y, (R)0);
-  }
+  return scale_w_entry<R, PK>(__ldg(reinterpret_cast<const typename ZposEntry<R>::type*>(tab) + site), up, x);
 }
 
 // x * (hi + lo), packed when PK (FP32 only)

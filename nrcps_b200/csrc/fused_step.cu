@@ -1193,10 +1193,20 @@ __global__ void __launch_bounds__(PullShape<R, L, C, false>::THREADS, PullShape<
         const uint64_t k0 = kb + (uint64_t)site0;
         const uint32_t* words = reinterpret_cast<const uint32_t*>(f.field) + (k0 >> 5);
         const int bit = (int)(k0 & 31);
+        // words and weights of a chunk of sites ahead of their use: FP64, L = 24, one
+        // orbital 20 us against 22, 627 148 against 159; FP32, L = 48, 627 801 against 848
+        constexpr int CH = sizeof(R) == 8 ? 4 : 8;
 #pragma unroll
-        for (int xx = 0; xx < L; ++xx) {
-          const bool up = (__ldg(words + xx * (L * L / 32)) >> bit) & 1u;
-          x[xx] = scale_w_zpos<R, PK>(f.zpos, site0 + xx * L * L, up, x[xx]);
+        for (int x0 = 0; x0 < L; x0 += CH) {
+          uint32_t word[CH];
+          typename ZposEntry<R>::type w[CH];
+#pragma unroll
+          for (int i = 0; i < CH; ++i) {
+            word[i] = __ldg(words + (x0 + i) * (L * L / 32));
+            w[i] = __ldg(reinterpret_cast<const typename ZposEntry<R>::type*>(f.zpos) + site0 + (x0 + i) * L * L);
+          }
+#pragma unroll
+          for (int i = 0; i < CH; ++i) x[x0 + i] = scale_w_entry<R, PK>(w[i], (word[i] >> bit) & 1u, x[x0 + i]);
         }
       } else if constexpr (FK == 2 || FK == 3) {
         if (AS::WT && wt) {
