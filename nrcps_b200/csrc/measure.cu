@@ -1011,10 +1011,10 @@ __global__ void __launch_bounds__(32 * kWarpLuMaxWarps) slater_dets_warp_kernel(
 // compared.
 //
 // Bound by the latency of a step (search, reciprocal, broadcast) at 16 warps
-// per SM and by instruction issue (49 %): 4096 matrices of N = 19 take 186 us
-// (a warp per minor in shared memory: 507; a warp per minor in registers, no
-// segments: 319), 4096 of N = 7 with struck columns 30 (130), 500 of N = 32
-// 153 (345).
+// per SM and by instruction issue (half of the cycles): 4096 matrices of N = 19
+// take 191 us (a warp per minor in shared memory: 504; a warp per minor in
+// registers, no segments: 319), 4096 of N = 7 with struck columns 30 (130), 500 of
+// N = 32 161 (346).
 constexpr int kRowLuWarps = 4;
 constexpr int kRowLuMax = 32;
 
@@ -1141,7 +1141,11 @@ __device__ __forceinline__ void minor_lu(const double2* __restrict__ S, const do
       for (int k = k4; k < k4 + 4; ++k) {
         if (k + 1 < NMAX) {
           const double2 w = u[k + 1];
-          a[k] = dc{fma(-l.re, w.x, fma(l.im, w.y, a[k + 1].re)), fma(-l.re, w.y, fma(-l.im, w.x, a[k + 1].im))};
+          // the product by itself, then one rounding at the entry's size: nested
+          // FMAs round there twice, 3 % less time and 1.4 times the error (rms over
+          // matrices 1 + 0.3 G of N = 19: 0.57e-15 against 0.41e-15, as before)
+          const dc p{fma(l.re, w.x, -(l.im * w.y)), fma(l.re, w.y, l.im * w.x)};
+          a[k] = dc{a[k + 1].re - p.re, a[k + 1].im - p.im};
         }
       }
     }
