@@ -410,7 +410,7 @@ def trapped_core(ctx, n_conf: int, steps: int, warmup: int, cpu_slices: int, pre
     e1.record()
     torch.cuda.synchronize()
     e2e_ms = e0.elapsed_time(e1) / steps
-    kind, cluster = ctx.fused_choice("f32", L)
+    kind, cluster = ctx.fused_choice("f32", L, n_conf * N)
     launches = ens.launches()
     ens.close()
     # the step's kernels alone on the same orbitals (FP32, n_conf x N)
@@ -553,7 +553,7 @@ def fp64_batched(a, ctx, idx, configs: int = 256):
         ens.run(k[0] * configs)
 
     ms = cuda_ms(run, 2)
-    kind, cluster = ctx.fused_choice("f64", a.L)
+    kind, cluster = ctx.fused_choice("f64", a.L, configs * len(idx))
     ens.close()
     return {"value": configs * a.T / (ms / 1000.0), "unit": UNIT, "ms_per_step": ms,
             "sample": f"{configs} configurations x {a.T} slices per step, L={a.L}^3 N={len(idx)}, FP64 orbitals and "
@@ -714,7 +714,7 @@ def run_b200(a):
     alg_bytes = 2.0 * a.L ** 3 * esize * rconf * n_orb
     achieved = alg_bytes / (kms / 1000.0) / 1e9
     peak, peak_src = hbm_peak()
-    kind, cluster = ctx.fused_choice(a.precision, a.L)
+    kind, cluster = ctx.fused_choice(a.precision, a.L, rconf * n_orb)
     traffic = NCU_TRAFFIC_PER_ORBITAL.get((a.precision, a.L, kind, cluster))
     roofline = {"bound": "hbm", "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
                 "frac": round(achieved / peak, 4),

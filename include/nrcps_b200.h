@@ -154,8 +154,12 @@ nrcps_status nrcps_autotune(nrcps_context *ctx, nrcps_precision prec, int L, int
  * variant serves the shape.  (13, 1) and (14, 1) name the kernels that hold an
  * orbital in one SM (FP32, L = 32) and in one CTA (L = 16): they run where no
  * variant is forced and the batch fills the device, or half of it; smaller
- * batches run a variant, with the same results.  Tunes nothing. */
+ * batches run a variant, with the same results.  The answer is that for large
+ * batches; nrcps_fused_choice_of gives the one for a step of n_orb orbitals
+ * (batch times configurations).  Tunes nothing. */
 nrcps_status nrcps_fused_choice(nrcps_context *ctx, nrcps_precision prec, int L, int *kind, int *cluster);
+nrcps_status nrcps_fused_choice_of(nrcps_context *ctx, nrcps_precision prec, int L, long n_orb, int *kind,
+                                   int *cluster);
 
 /* ----------------------------------------------------- host-side tables
  * Replace the reference's host constructors' table builds so that callers

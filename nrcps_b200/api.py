@@ -90,10 +90,12 @@ class Context:
         self.check(lib().nrcps_autotune(self.handle, _prec(precision), L, ctypes.byref(c)), "autotune")
         return c.value
 
-    def fused_choice(self, precision: str, L: int):
-        """(kind, cluster) of the fused kernel nrcps_propagate runs for (precision, L^3); (-1, -1) if none."""
+    def fused_choice(self, precision: str, L: int, orbitals: Optional[int] = None):
+        """(kind, cluster) of the fused kernel nrcps_propagate runs for (precision, L^3) and this many
+        orbitals (None: a large batch); (-1, -1) if none."""
         k, c = ctypes.c_int(), ctypes.c_int()
-        self.check(lib().nrcps_fused_choice(self.handle, _prec(precision), L, ctypes.byref(k), ctypes.byref(c)),
+        n = 1 << 20 if orbitals is None else orbitals
+        self.check(lib().nrcps_fused_choice_of(self.handle, _prec(precision), L, n, ctypes.byref(k), ctypes.byref(c)),
                    "fused_choice")
         return k.value, c.value
 

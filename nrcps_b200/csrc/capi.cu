@@ -119,7 +119,7 @@ extern "C" nrcps_status nrcps_set_stream(nrcps_context* ctx, void* stream) {
 
 namespace nrcps {
 nrcps_status fused_autotune(nrcps_context* ctx, nrcps_precision prec, int L, int* chosen_cluster);
-nrcps_status fused_choice(nrcps_context* ctx, nrcps_precision prec, int L, int* kind, int* cluster);
+nrcps_status fused_choice(nrcps_context* ctx, nrcps_precision prec, int L, long n_orb, int* kind, int* cluster);
 }
 
 extern "C" nrcps_status nrcps_set_option(nrcps_context* ctx, const char* name, long value) {
@@ -168,9 +168,14 @@ extern "C" nrcps_status nrcps_autotune(nrcps_context* ctx, nrcps_precision prec,
 }
 
 extern "C" nrcps_status nrcps_fused_choice(nrcps_context* ctx, nrcps_precision prec, int L, int* kind, int* cluster) {
-  if (!ctx || !kind || !cluster || L <= 0) return NRCPS_ERR_INVALID_ARGUMENT;
+  return nrcps_fused_choice_of(ctx, prec, L, 1L << 20, kind, cluster);
+}
+
+extern "C" nrcps_status nrcps_fused_choice_of(nrcps_context* ctx, nrcps_precision prec, int L, long n_orb, int* kind,
+                                              int* cluster) {
+  if (!ctx || !kind || !cluster || L <= 0 || n_orb < 0) return NRCPS_ERR_INVALID_ARGUMENT;
   if (prec != NRCPS_F32 && prec != NRCPS_F64) return set_error(ctx, NRCPS_ERR_INVALID_ARGUMENT, "bad precision");
-  return fused_choice(ctx, prec, L, kind, cluster);
+  return fused_choice(ctx, prec, L, n_orb, kind, cluster);
 }
 
 // Waits for the context's stream, then reports a timed-out bounded wait in

@@ -1677,10 +1677,10 @@ static int fused_whole_kind(nrcps_context* ctx, nrcps_precision prec, int L, int
   return 3 * n_orb > 2 * waves * slots ? 13 : 0;
 }
 
-nrcps_status fused_choice(nrcps_context* ctx, nrcps_precision prec, int L, int* kind, int* cluster) {
+nrcps_status fused_choice(nrcps_context* ctx, nrcps_precision prec, int L, long n_orb, int* kind, int* cluster) {
   const int d[3] = {L, L, L};
-  const int whole = ctx->fused_enabled ? fused_whole_kind(ctx, prec, L, ctx->fused_cluster, 1L << 20) : 0;
-  if (whole) {  // (large batches)
+  const int whole = ctx->fused_enabled ? fused_whole_kind(ctx, prec, L, ctx->fused_cluster, n_orb) : 0;
+  if (whole) {
     *kind = whole;
     *cluster = 1;
     return NRCPS_OK;
