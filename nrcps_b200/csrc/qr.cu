@@ -21,29 +21,28 @@ namespace nrcps {
 bool gram_tc_supported(int N, long vol, int nconf);
 nrcps_status gram_tc(nrcps_context* ctx, const void* psi, int N, long vol, int nconf, double* G);
 
-// FP64 orbitals: G[c][i][j] for i <= j (the upper triangle the Cholesky reads), one block
-// per configuration reading its orbitals once: tiles of GT sites of all N
+// FP64 orbitals: G[c][i][j] for i <= j (the upper triangle the Cholesky reads), one
+// block per configuration reading its orbitals once: tiles of GT sites of all N
 // orbitals go through shared memory (rows padded by one element so that the
 // rows a warp reads fall in different banks); each thread accumulates 2 x 2
-// blocks (i, i+1) x (j, j+1) of G over a quarter of each tile's sites, in R
-// within a tile and in FP64 across tiles; the four quarters are summed at
-// the end.
+// blocks (i, i+1) x (j, j+1) of G over a quarter of each tile's sites, a tile's
+// sums apart; the four quarters are summed at the end.
 constexpr int GT = 128;
-__device__ __forceinline__ void cp_async_elem(void* dst, const void* src, int bytes) {
-  const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
-  if (bytes == 16) asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
-  else asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(d), "l"(src) : "memory");
+__device__ __forceinline__ void cp_async_elem(cplx<double>* dst, const cplx<double>* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
+               : "memory");
 }
 
 // DB: double-buffered tiles (the next tile's asynchronous copies overlap the
 // current tile's products); else one tile buffer.
-template <typename R, int MAXB, bool DB = false>
+template <int MAXB, bool DB>
 __global__ void __launch_bounds__(256) gram_tile_kernel(const void* __restrict__ psi, int N, long vol,
                                                         double* __restrict__ G) {
+  typedef cplx<double> cd;
   extern __shared__ __align__(16) unsigned char gsm[];
-  cplx<R>* tiles = reinterpret_cast<cplx<R>*>(gsm);  // [DB ? 2 : 1][N][GT + 1]
+  cd* tiles = reinterpret_cast<cd*>(gsm);  // [DB ? 2 : 1][N][GT + 1]
   const long c = blockIdx.x;
-  const cplx<R>* base = reinterpret_cast<const cplx<R>*>(psi) + (size_t)c * N * vol;
+  const cd* base = reinterpret_cast<const cd*>(psi) + (size_t)c * N * vol;
   const int nb = (N + 1) / 2;                // 2-row blocks
   const int nblk = nb * (nb + 1) / 2;        // upper-triangular block pairs
   const int lane64 = threadIdx.x & 63, grp = threadIdx.x >> 6;
@@ -53,12 +52,12 @@ __global__ void __launch_bounds__(256) gram_tile_kernel(const void* __restrict__
   for (int b = 0; b < MAXB; ++b)
 #pragma unroll
     for (int k = 0; k < 8; ++k) acc[b][k] = 0.0;
-  auto fill = [&](long p0, cplx<R>* t) {
+  auto fill = [&](long p0, cd* t) {
     const int ts = (int)((vol - p0) < GT ? (vol - p0) : GT);
     for (int e = threadIdx.x; e < N * GT; e += blockDim.x) {
       const int i = e / GT, s = e - i * GT;
-      if (!DB || s >= ts) t[i * (GT + 1) + s] = s < ts ? base[(size_t)i * vol + p0 + s] : cplx<R>{(R)0, (R)0};
-      else cp_async_elem(t + i * (GT + 1) + s, base + (size_t)i * vol + p0 + s, (int)sizeof(cplx<R>));
+      if (!DB || s >= ts) t[i * (GT + 1) + s] = s < ts ? base[(size_t)i * vol + p0 + s] : cd{0.0, 0.0};
+      else cp_async_elem(t + i * (GT + 1) + s, base + (size_t)i * vol + p0 + s);
     }
     if (DB) asm volatile("cp.async.commit_group;" ::: "memory");
   };
@@ -66,7 +65,7 @@ __global__ void __launch_bounds__(256) gram_tile_kernel(const void* __restrict__
   if (DB) fill(0, tiles);
   int buf = 0;
   for (long p0 = 0; p0 < vol; p0 += GT, buf ^= 1) {
-    cplx<R>* tile = tiles + (DB ? buf : 0) * tsz;
+    cd* tile = tiles + (DB ? buf : 0) * tsz;
     if (DB) {
       __syncthreads();  // every thread is done with the tile the next copies overwrite
       if (p0 + GT < vol) fill(p0 + GT, tiles + (buf ^ 1) * tsz);
@@ -91,12 +90,12 @@ __global__ void __launch_bounds__(256) gram_tile_kernel(const void* __restrict__
       const int bj = bi + rem;
       const int i0 = 2 * bi, j0 = 2 * bj;
       const int i1 = i0 + 1 < N ? i0 + 1 : i0, j1 = j0 + 1 < N ? j0 + 1 : j0;
-      R s[8];
+      double s[8];
 #pragma unroll
-      for (int k = 0; k < 8; ++k) s[k] = (R)0;
+      for (int k = 0; k < 8; ++k) s[k] = 0.0;
       for (int q = grp; q < GT; q += 4) {
-        const cplx<R> a0 = tile[i0 * (GT + 1) + q], a1 = tile[i1 * (GT + 1) + q];
-        const cplx<R> b0 = tile[j0 * (GT + 1) + q], b1 = tile[j1 * (GT + 1) + q];
+        const cd a0 = tile[i0 * (GT + 1) + q], a1 = tile[i1 * (GT + 1) + q];
+        const cd b0 = tile[j0 * (GT + 1) + q], b1 = tile[j1 * (GT + 1) + q];
         // conj(a) b: two fused multiply-adds per component
         s[0] = fma(a0.re, b0.re, s[0]);
         s[0] = fma(a0.im, b0.im, s[0]);
@@ -116,7 +115,7 @@ __global__ void __launch_bounds__(256) gram_tile_kernel(const void* __restrict__
         s[7] = fma(-a1.im, b1.re, s[7]);
       }
 #pragma unroll
-      for (int k = 0; k < 8; ++k) acc[b][k] += (double)s[k];
+      for (int k = 0; k < 8; ++k) acc[b][k] += s[k];
     }
   }
   // sum the four site quarters through shared memory, write the upper triangle
@@ -627,6 +626,22 @@ static nrcps_status launch_gram4(nrcps_context* ctx, const void* psi, int N, lon
                     "gram4_kernel");
 }
 
+static nrcps_status launch_gram_tile(nrcps_context* ctx, const void* psi, int N, long vol, int nconf, double* G) {
+  const size_t tile_bytes = sizeof(cplx<double>) * (size_t)N * (GT + 1);
+  const bool db = 2 * tile_bytes <= 200 * 1024;
+  size_t sh = db ? 2 * tile_bytes : tile_bytes;
+  const size_t red = sizeof(double) * 8 * 528;
+  if (sh < red) sh = red;
+  auto launch = [&](auto kern) -> nrcps_status {
+    NRCPS_TRY(allow_smem(ctx, (const void*)kern, 200 * 1024, "gram_tile_kernel: smem attribute"));
+    kern<<<(unsigned)nconf, 256, sh, ctx->stream>>>(psi, N, vol, G);
+    return check_launch(ctx, "gram_tile_kernel");
+  };
+  if (N <= 22) return launch(gram_tile_kernel<2, true>);
+  if (N <= 32) return launch(gram_tile_kernel<3, true>);
+  return db ? launch(gram_tile_kernel<9, true>) : launch(gram_tile_kernel<9, false>);
+}
+
 // One re-orthonormalisation of nconf configurations of N orbitals.
 // G: scratch of nconf * N * N complex doubles; logR accumulates.
 nrcps_status qr_reorthonormalise(nrcps_context* ctx, void* psi, int N, long vol, int nconf, nrcps_precision prec,
@@ -635,26 +650,8 @@ nrcps_status qr_reorthonormalise(nrcps_context* ctx, void* psi, int N, long vol,
   if (prec == NRCPS_F32 && ctx->qr_gram_tc && gram_tc_supported(N, vol, nconf)) {
     NRCPS_TRY(gram_tc(ctx, psi, N, vol, nconf, G));  // tcgen05, TF32 hi/lo (gram_tc.cu)
   } else {
-    const size_t esz = prec == NRCPS_F64 ? sizeof(cplx<double>) : sizeof(cplx<float>);
-    const size_t tile_bytes = esz * (size_t)N * (GT + 1);
-    const bool db = 2 * tile_bytes <= 200 * 1024;
-    size_t sh = db ? 2 * tile_bytes : tile_bytes;
-    const size_t red = sizeof(double) * 8 * 528;
-    if (sh < red) sh = red;
-    auto launch = [&](auto kern) {
-      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-      kern<<<(unsigned)nconf, 256, sh, ctx->stream>>>(psi, N, vol, G);
-    };
-    if (prec == NRCPS_F64) {
-      if (N <= 22) launch(gram_tile_kernel<double, 2, true>);
-      else if (N <= 32) launch(gram_tile_kernel<double, 3, true>);
-      else if (db) launch(gram_tile_kernel<double, 9, true>);
-      else launch(gram_tile_kernel<double, 9, false>);
-    } else {
-      NRCPS_TRY(launch_gram4(ctx, psi, N, vol, nconf, G));
-    }
+    NRCPS_TRY(prec == NRCPS_F64 ? launch_gram_tile(ctx, psi, N, vol, nconf, G) : launch_gram4(ctx, psi, N, vol, nconf, G));
     ctx->launches++;
-    NRCPS_TRY(check_launch(ctx, "gram_tile_kernel"));
   }
   const size_t chol_sh = sizeof(double2) * N * N;
   if (chol_sh > 48 * 1024)
