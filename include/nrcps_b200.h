@@ -153,8 +153,9 @@ nrcps_status nrcps_autotune(nrcps_context *ctx, nrcps_precision prec, int L, int
  * "fused.kind") and *cluster (CTAs per cluster); both -1 when no fused
  * variant serves the shape.  (13, 1) and (14, 1) name the kernels that hold an
  * orbital in one SM (FP32, L = 32) and in one CTA (L = 16): they run where no
- * variant is forced and the batch fills the device, or half of it; smaller
- * batches run a variant, with the same results.  The answer is that for large
+ * variant is forced and the batch fills the device (at L = 16 an eighth of it;
+ * the step of a Z2 field with a position factor at L = 32 seven eighths of its
+ * last round of orbitals); smaller batches run a variant, with the same results.  The answer is that for large
  * batches; nrcps_fused_choice_of gives the one for a step of n_orb orbitals
  * (batch times configurations).  Tunes nothing. */
 nrcps_status nrcps_fused_choice(nrcps_context *ctx, nrcps_precision prec, int L, int *kind, int *cluster);

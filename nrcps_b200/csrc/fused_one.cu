@@ -100,9 +100,19 @@ __global__ void __launch_bounds__(OneShape<R>::THREADS, OneShape<R>::CTAS) fused
         const uint32_t* words = reinterpret_cast<const uint32_t*>(f.field) + (k0 >> 5);
         const int bit = (int)(k0 & 31);
         if (f.zpos) {
+          constexpr int CH = 4;  // words and weights of four sites ahead of their use
 #pragma unroll
-          for (int xx = 0; xx < L; ++xx)
-            x[xx] = scale_w_zpos<R, false>(f.zpos, p + xx * L * L, (__ldg(words + xx * (L * L / 32)) >> bit) & 1u, x[xx]);
+          for (int x0 = 0; x0 < L; x0 += CH) {
+            uint32_t word[CH];
+            typename ZposEntry<R>::type w[CH];
+#pragma unroll
+            for (int i = 0; i < CH; ++i) {
+              word[i] = __ldg(words + (x0 + i) * (L * L / 32));
+              w[i] = __ldg(reinterpret_cast<const typename ZposEntry<R>::type*>(f.zpos) + p + (x0 + i) * L * L);
+            }
+#pragma unroll
+            for (int i = 0; i < CH; ++i) x[x0 + i] = scale_w_entry<R, false>(w[i], (word[i] >> bit) & 1u, x[x0 + i]);
+          }
         } else if (w_exact) {
 #pragma unroll
           for (int xx = 0; xx < L; ++xx) {

@@ -1661,25 +1661,27 @@ bool fused_admits(nrcps_context* ctx, nrcps_precision prec, const int d[3]) {
 // an orbital per CTA, `slots` at a time (kind 13: 26 us each at 19456
 // orbitals, 0.182 us per orbital against 0.246 for kind 11, cluster 8, which
 // spreads an orbital over 8 CTAs, 74 at a time).  Kind 13 pays where its last
-// wave is not mostly empty, kind 14, which has several CTAs per SM, from half a
-// wave on.  Measured, kind 13 against kind 11: 57 orbitals 32 / 26
-// us, 95 35 / 37, 152 61 / 50, 190 61 / 58, 304 87 / 85, 988 224 / 258, 19456
-// 3544 / 4778; kind 14, FP64 (444 slots) against kind 0, cluster 2: 300
-// orbitals 17 / 20 us, 444 17 / 23, 600 25 / 31, 3500 131 / 161; FP32 (888
-// slots) against kind 11, cluster 2: 600 18 / 27, 2100 42 / 53.
-static int fused_whole_kind(nrcps_context* ctx, nrcps_precision prec, int L, int cluster, long n_orb) {
+// wave is not mostly empty, nearly full where each of its orbitals reads the weights
+// of a Z2 field with a potential (512 KB) from L2 by itself; kind 14, which has
+// several CTAs per SM, from an eighth of a wave on.  Measured, kind 13 against kind
+// 11: 57 orbitals 32 / 26 us, 95 35 / 37, 152 61 / 50, 190 61 / 58, 304 87 / 85, 330
+// 89 / 96, 988 224 / 258, 19456 3544 / 4778; with a potential 210 72 / 69, 304 99 /
+// 93, 600 183 / 171, 260 72 / 83, 440 109 / 129; kind 14, FP64 (444 slots) against
+// kind 0, cluster 2: 100 orbitals 9.4 / 12.5 us, 152 12.4 / 14.0, 444 17 / 23, 3500
+// 131 / 161; FP32 (888 slots) against kind 11, cluster 2: 57 orbitals 11.5 / 11.5
+// (Gaussian field 13.5 / 11.5), 140 11.5 / 13.5, 304 15.5 / 19.6, 2100 42 / 53.
+static int fused_whole_kind(nrcps_context* ctx, nrcps_precision prec, int L, int cluster, long n_orb, bool weights) {
   if (cluster > 0 || ctx->fused_split >= 0 || ctx->fused_kind >= 0) return 0;
-  const bool park = L == 32;
   const long slots = whole_slots(ctx, prec, L);
   if (slots == 0) return 0;
-  if (!park) return 2 * n_orb > slots ? 14 : 0;
+  if (L != 32) return 8 * n_orb > slots ? 14 : 0;
   const long waves = (n_orb + slots - 1) / slots;
-  return 3 * n_orb > 2 * waves * slots ? 13 : 0;
+  return (weights ? 8 * n_orb > 7 * waves * slots : 3 * n_orb > 2 * waves * slots) ? 13 : 0;
 }
 
 nrcps_status fused_choice(nrcps_context* ctx, nrcps_precision prec, int L, long n_orb, int* kind, int* cluster) {
   const int d[3] = {L, L, L};
-  const int whole = ctx->fused_enabled ? fused_whole_kind(ctx, prec, L, ctx->fused_cluster, n_orb) : 0;
+  const int whole = ctx->fused_enabled ? fused_whole_kind(ctx, prec, L, ctx->fused_cluster, n_orb, false) : 0;
   if (whole) {
     *kind = whole;
     *cluster = 1;
@@ -1724,7 +1726,7 @@ nrcps_status fused_step(nrcps_context* ctx, void* psi, int batch, int nconf, con
   f.wait_ns = ctx->fused_wait_ns;
   f.stall_test = ctx->fused_stall_test;
   if (f.n_orb_total == 0) return NRCPS_OK;
-  switch (fused_whole_kind(ctx, prec, d[0], cluster, f.n_orb_total)) {
+  switch (fused_whole_kind(ctx, prec, d[0], cluster, f.n_orb_total, f.zpos != nullptr)) {
     case 13: return fused_park_step(ctx, f);
     case 14: return fused_one_step(ctx, prec, f);
   }

@@ -19,10 +19,10 @@ def _sms():
 
 
 @pytest.mark.parametrize("precision,per_sm", [("f64", 3), ("f32", 6)])
-def test_one_cta_kernel_from_half_a_wave(ctx, precision, per_sm):
-    half = _sms() * per_sm // 2
-    assert ctx.fused_choice(precision, 16, half)[0] not in (13, 14)
-    for n in (half + 1, 2 * half, 2 * half + 1, 1 << 20, None):
+def test_one_cta_kernel_from_an_eighth_of_a_wave(ctx, precision, per_sm):
+    slots = _sms() * per_sm
+    assert ctx.fused_choice(precision, 16, slots // 8)[0] not in (13, 14)
+    for n in (slots // 8 + 1, slots // 2, slots, slots + 1, 1 << 20, None):
         assert ctx.fused_choice(precision, 16, n) == (14, 1)
 
 
