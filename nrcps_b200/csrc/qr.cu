@@ -165,20 +165,21 @@ __global__ void __launch_bounds__(256) gram_tile_kernel(const void* __restrict__
 // each row of the inverse by one thread per column.  A serial chain of N
 // square roots and divisions is left: 29 us for 256 matrices of N = 19, 34 us
 // for 1024 (one thread per matrix: 610 and 675 us).
-constexpr int CHOL_THREADS = 128;
+constexpr int CHOL_THREADS = 128;  // a warp for N <= 8
 __global__ void __launch_bounds__(CHOL_THREADS) chol_inv_kernel(double* __restrict__ G, int N,
                                                                 double* __restrict__ logR, int f32_apply) {
   extern __shared__ double2 cm[];  // [N][N]
   const long c = blockIdx.x;
+  const int threads = (int)blockDim.x;
   double* g = G + 2 * c * N * N;  // (the caller's work buffer: doubles, not on 16 bytes of need)
   auto write_back = [&]() {
-    for (int e = threadIdx.x; e < N * N; e += CHOL_THREADS)
+    for (int e = threadIdx.x; e < N * N; e += threads)
       if (e / N <= e % N) {
         g[2 * e] = cm[e].x;
         g[2 * e + 1] = cm[e].y;
       }
   };
-  for (int e = threadIdx.x; e < N * N; e += CHOL_THREADS)
+  for (int e = threadIdx.x; e < N * N; e += threads)
     if (e / N <= e % N) cm[e] = make_double2(g[2 * e], g[2 * e + 1]);
   __syncthreads();
   bool ok = true;
@@ -190,14 +191,14 @@ __global__ void __launch_bounds__(CHOL_THREADS) chol_inv_kernel(double* __restri
     }
     const double rkk = sqrt(d);
     __syncthreads();  // every thread has read the pivot
-    for (int j = k + threadIdx.x; j < N; j += CHOL_THREADS) {
+    for (int j = k + threadIdx.x; j < N; j += threads) {
       if (j == k) cm[k * N + k] = make_double2(rkk, 0.0);
       else cm[k * N + j] = make_double2(cm[k * N + j].x / rkk, cm[k * N + j].y / rkk);
     }
     __syncthreads();
     // G_ij -= conj(R_ki) R_kj for k < i <= j
     const int m = N - k - 1;
-    for (int e = threadIdx.x; e < m * m; e += CHOL_THREADS) {
+    for (int e = threadIdx.x; e < m * m; e += threads) {
       const int i = k + 1 + e / m, j = k + 1 + e % m;
       if (i > j) continue;
       const double2 a = cm[k * N + i], b = cm[k * N + j];
@@ -214,15 +215,15 @@ __global__ void __launch_bounds__(CHOL_THREADS) chol_inv_kernel(double* __restri
   }
   if (!ok) {
     write_back();
-    for (int i = threadIdx.x; i < N; i += CHOL_THREADS) logR[c * N + i] = nan("");
+    for (int i = threadIdx.x; i < N; i += threads) logR[c * N + i] = nan("");
     return;
   }
   if (!f32_apply)
-    for (int i = threadIdx.x; i < N; i += CHOL_THREADS) logR[c * N + i] += log(cm[i * N + i].x);
+    for (int i = threadIdx.x; i < N; i += threads) logR[c * N + i] += log(cm[i * N + i].x);
   __syncthreads();
   // Rinv in place, row by row from the bottom: Rinv_ii = 1 / R_ii,
   // Rinv_ij = -(sum_{k=i+1..j} R_ik Rinv_kj) / R_ii for j > i (a thread per j;
-  // N <= 64 < CHOL_THREADS)
+  // N is at most the threads)
   for (int i = N - 1; i >= 0; --i) {
     const double rii = cm[i * N + i].x;
     const int j = i + 1 + threadIdx.x;
@@ -239,7 +240,7 @@ __global__ void __launch_bounds__(CHOL_THREADS) chol_inv_kernel(double* __restri
     __syncthreads();
   }
   if (f32_apply)
-    for (int i = threadIdx.x; i < N; i += CHOL_THREADS) logR[c * N + i] -= log((double)(float)cm[i * N + i].x);
+    for (int i = threadIdx.x; i < N; i += threads) logR[c * N + i] -= log((double)(float)cm[i * N + i].x);
   write_back();
 }
 
@@ -393,11 +394,23 @@ __global__ void __launch_bounds__(G4_THREADS, 2) gram4_kernel(const float2* __re
   __syncthreads();
   // the lanes and groups of every pair, then the cluster's CTAs
   double* red = reinterpret_cast<double*>(tiles);  // [here][32], over the stages
+  static_assert(groups <= 2 || sizeof(double) * npairs * 32 * (G4_LANES + 1) <= sizeof(float) * 4 * plane, "sums over the stages");
+  if (groups > 2) {  // the groups of an entry and lane first, by all threads (256 sums in a row took 3 us)
+    double* lanes = red + here * 32;  // [here][32][G4_LANES]
+    for (int e = threadIdx.x; e < here * 32 * G4_LANES; e += G4_THREADS) {
+      const int j = e % G4_LANES, k = e / G4_LANES % 32, pr = e / G4_LANES / 32;
+      double v = 0.0;
+      for (int g = 0; g < groups; ++g) v += acc[k * G4_THREADS + (g * here + pr) * G4_LANES + j];
+      lanes[e] = v;
+    }
+    __syncthreads();
+  }
   for (int e = threadIdx.x; e < here * 32; e += G4_THREADS) {
     const int pr = e / 32, k = e % 32;
+    const double* from = groups > 2 ? red + here * 32 + e * G4_LANES : acc + k * G4_THREADS + pr * G4_LANES;
     double v = 0.0;
-    for (int g = 0; g < groups; ++g)
-      for (int j = 0; j < G4_LANES; ++j) v += acc[k * G4_THREADS + (g * here + pr) * G4_LANES + j];
+    for (int g = 0; g < (groups > 2 ? 1 : groups); ++g)
+      for (int j = 0; j < G4_LANES; ++j) v += from[g * here * G4_LANES + j];
     red[e] = v;
   }
   cluster.sync();
@@ -656,7 +669,7 @@ nrcps_status qr_reorthonormalise(nrcps_context* ctx, void* psi, int N, long vol,
   const size_t chol_sh = sizeof(double2) * N * N;
   if (chol_sh > 48 * 1024)
     NRCPS_TRY(allow_smem(ctx, (const void*)chol_inv_kernel, kMatrixSmem, "chol_inv_kernel: smem attribute"));
-  chol_inv_kernel<<<(unsigned)nconf, CHOL_THREADS, chol_sh, ctx->stream>>>(G, N, logR, prec == NRCPS_F32);
+  chol_inv_kernel<<<(unsigned)nconf, N <= 8 ? 32 : CHOL_THREADS, chol_sh, ctx->stream>>>(G, N, logR, prec == NRCPS_F32);
   ctx->launches++;
   NRCPS_TRY(check_launch(ctx, "chol_inv_kernel"));
   if (N <= 8) return launch_apply<8>(ctx, psi, N, vol, nconf, prec, G);
