@@ -5,8 +5,10 @@
 #include <stdint.h>
 
 #include <cstdio>
+#include <map>
 #include <string>
 #include <unordered_map>
+#include <utility>
 
 #include "../../include/nrcps_b200.h"
 
@@ -117,6 +119,7 @@ struct Context {
   // Kernels whose attributes this context has set, and for the clustered ones
   // how many clusters fit the device (allow_smem, launch_fused).
   std::unordered_map<const void*, int> kernels;
+  std::map<std::pair<const void*, int>, int> clusters;  // (kernel, CTAs of a cluster): clusters that fit (pair_sym.cu)
   void* overlap_part = nullptr;  // chunk sums of the CUDA-core overlap (fixed size, made at the first use)
   cudaEvent_t overlap_done = nullptr;  // the last use of overlap_part, waited for by the next
   int* dev_err = nullptr;

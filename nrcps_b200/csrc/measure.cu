@@ -1485,7 +1485,7 @@ static nrcps_status launch_pair_tile(nrcps_context* ctx, const void* psi1, const
   return check_cuda(ctx, e, "pair_tile_kernel launch");
 }
 
-bool pair_sym_supported(int n);  // pair_sym.cu
+bool pair_sym_supported(int n, long vol);  // pair_sym.cu
 nrcps_status pair_sym(nrcps_context* ctx, const void* psi, int n, int nconf, long vol, const double* w, const int* opp,
                       const int* flags, double* phi);
 
@@ -1508,7 +1508,7 @@ nrcps_status pair_impl(nrcps_context* ctx, const void* psi1, const void* psi2, i
       return launch_pair_tile<double>(ctx, psi1, psi2, n, nconf, vol, w, opp, flags, props, false, phi);
     // one set of FP32 orbitals: the packed kernel where the table qualifies;
     // a table checked on the device decides there which of the two runs
-    const bool one_set = psi1 == psi2 && pair_sym_supported(n);
+    const bool one_set = psi1 == psi2 && pair_sym_supported(n, vol);
     if (one_set && (flags || !props)) {
       NRCPS_TRY(pair_sym(ctx, psi1, n, nconf, vol, w, opp, flags, phi));
       if (!flags) return NRCPS_OK;

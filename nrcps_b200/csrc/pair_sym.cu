@@ -17,21 +17,21 @@
 // Operands stay as (re, im) pairs: P += a . b and Q += a . swap(b)
 // (elementwise, packed FP32x2) hold the four real sums, re phi = P.x - P.y, im
 // phi = Q.x + Q.y, so that a product costs two packed FMAs and only b is
-// swapped.  Every six pairs of sites (12 terms) the lanes of a warp add their
-// sums up over a reduce-scatter of shuffles and each takes two of the 50 into
-// FP64: two conversions where a lane's own sums would take 50.  A level of the
-// tree rounds every sum once; sums of six pairs keep the error against 64 bits
-// at that of the general kernel, whose chains are 15 terms at n = 10 (L = 48,
-// n = 10: 1.03e-7 against 1.06e-7 relative; sums of eight: 1.18e-7).
+// swapped.  Every four pairs of sites (8 terms) groups of eight lanes of a warp
+// add their sums up over three levels of a reduce-scatter of shuffles and each
+// lane takes eight of the 50 into FP64, where the last two levels follow at the
+// end: eight conversions where a lane's own sums would take 50.  A level of the
+// tree rounds every sum once, at its whole size where the terms are of one sign
+// (orbitals without nodes).  Short sums and three levels keep the error against 64
+// bits at or below that of the general kernel, whose chains are 15 terms at n =
+// 10, for orbitals of random sign and for positive ones alike; six pairs and five
+// levels had 1.8 times its error on positive orbitals (n = 10, L = 24).
 //
 // What bounds it: at L = 48, n = 10, 128 configurations one read of the
-// orbitals takes 173 us and the FMAs 137; measured 400 us (the general kernel,
-// 2 x 2 blocks a thread through shared memory: 1012).  An instruction issues
-// in 42 % of the cycles: about ten warps per SM (168 registers) wait in turn
-// for a tile's copies, the barrier and their own FMAs; the reduce-scatter is a
-// quarter of the instructions.  Tiles of 64 sites in six stages: 507 us; three
-// of the five tree levels, the rest in FP64: 431.  n = 19, L = 32, 256
-// configurations: 0.81 ms against 1.20.
+// orbitals takes 173 us and the FMAs 137; measured 440 us (the general kernel,
+// 2 x 2 blocks a thread through shared memory: 1012; six pairs and five levels
+// 400).  About ten warps per SM (168 registers) wait in turn for a tile's copies,
+// the barrier and their own FMAs.  Tiles of 64 sites in six stages: 507 us.
 #include <cooperative_groups.h>
 
 #include "lane_sums.cuh"
@@ -45,7 +45,8 @@ constexpr int SB = 5;           // rows of a block
 constexpr int ST = 128;         // sites of a tile
 constexpr int SUNITS = ST / 32;
 constexpr int SSTAGES = 3;
-constexpr int SFLUSH = 6;       // pairs of sites of one FP32 sum
+constexpr int SFLUSH = 4;       // pairs of sites of one FP32 sum
+constexpr int SLEVELS = 3;      // levels of the lanes' tree in FP32
 constexpr int SWINDOW = 256;    // tiles whose bits are looked up at a time
 
 // NB blocks of rows: warps [0, NB) own the diagonal, the others the blocks
@@ -73,7 +74,7 @@ __device__ __forceinline__ void copy8(void* dst, const void* src, bool take) {
 // A warp's block: all 25 entries, or the 15 of the triangle (DIAG).
 struct SymAcc {
   float2 P[SB * SB], Q[SB * SB];
-  double sum[lane_share(2 * SB * SB)];
+  double sum[64 >> SLEVELS];
   int count;
   template <bool DIAG>
   static __host__ __device__ constexpr int entries() {
@@ -112,10 +113,16 @@ struct SymAcc {
       v[2 * e] = P[e].x - P[e].y;
       v[2 * e + 1] = Q[e].x + Q[e].y;
     }
-    reduce_scatter<2 * entries<DIAG>()>(v, lane);
+    reduce_scatter<2 * entries<DIAG>(), 0, SLEVELS>(v, lane);
 #pragma unroll
-    for (int k = 0; k < lane_share(2 * entries<DIAG>()); ++k) sum[k] += (double)v[k];
+    for (int k = 0; k < 32 * lane_share(2 * entries<DIAG>()) >> SLEVELS; ++k) sum[k] += (double)v[k];
     clear();
+  }
+  // the lanes' FP64 sums over the levels that are left
+  template <bool DIAG>
+  __device__ __forceinline__ void finish(int lane) {
+    flush<DIAG>(lane);
+    reduce_scatter<2 * entries<DIAG>(), SLEVELS, 5>(sum, lane);
   }
 };
 
@@ -278,8 +285,8 @@ __global__ void __launch_bounds__(SymShape<NB>::THREADS, SymShape<NB>::CTAS)
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
   }
-  if (diag) acc.flush<true>(lane);
-  else acc.flush<false>(lane);
+  if (diag) acc.finish<true>(lane);
+  else acc.finish<false>(lane);
   __syncthreads();
   // every warp's sums over the stages, then the cluster's CTAs in rank order
   double* red = reinterpret_cast<double*>(ssm);  // [WARPS][64]
@@ -307,18 +314,50 @@ __global__ void __launch_bounds__(SymShape<NB>::THREADS, SymShape<NB>::CTAS)
   cluster.sync();  // peers keep their shared memory until every sum is read
 }
 
+// Clusters of `split` CTAs of a kernel that the device runs at a time, asked of the
+// driver once per context (its occupancy query takes a few microseconds).
+nrcps_status clusters_that_fit(nrcps_context* ctx, const void* kern, int split, int threads, size_t smem, int per_sm,
+                               int* fit) {
+  int& known = ctx->clusters[{kern, split}];
+  if (known) {
+    *fit = known;
+    return NRCPS_OK;
+  }
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = (unsigned)split;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cfg.gridDim = dim3((unsigned)(split * ctx->sm_count));
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  if (cudaOccupancyMaxActiveClusters(fit, kern, &cfg) != cudaSuccess || *fit < 1) {
+    cudaGetLastError();
+    *fit = ctx->sm_count * per_sm / split;
+    if (*fit < 1) *fit = 1;
+  }
+  known = *fit;
+  return NRCPS_OK;
+}
+
 template <int NB>
 nrcps_status launch_pair_sym(nrcps_context* ctx, const void* psi, int n, int nconf, long vol, const double* w,
                              const int* opp, const int* flags, double* phi) {
   using Sh = SymShape<NB>;
   auto kern = pair_sym_kernel<NB>;
   NRCPS_TRY(allow_smem(ctx, (const void*)kern, Sh::SMEM, "pair_sym: smem attribute"));
-  // the split of a configuration that leaves the fewest rounds of CTAs per share
-  const long slots = (long)ctx->sm_count * Sh::CTAS, ntiles = (vol + ST - 1) / ST;
+  // the split of a configuration that leaves the fewest rounds of clusters per
+  // share, of as many clusters as fit the device (fewer than its SMs divided by
+  // the split: a GPC's SMs do not divide by every split)
+  const long ntiles = (vol + ST - 1) / ST;
   int split = 1;
   double best = 1e300;
   for (int s = 1; s <= 8 && s <= ntiles; ++s) {
-    const double cost = (double)((nconf * (long)s + slots - 1) / slots) / s;
+    int fit = 0;
+    NRCPS_TRY(clusters_that_fit(ctx, (const void*)kern, s, Sh::THREADS, Sh::SMEM, Sh::CTAS, &fit));
+    const double cost = (double)((nconf + fit - 1) / fit) / s;
     if (cost < 0.97 * best) best = cost, split = s;
   }
   cudaLaunchConfig_t cfg = {};
@@ -341,9 +380,15 @@ nrcps_status launch_pair_sym(nrcps_context* ctx, const void* psi, int n, int nco
 }  // namespace
 
 // Below n = 9 the general kernel's chains are short (10 terms at n = 8) and its
-// error 10 % less than this kernel's; at 11 and 12 also, and three blocks of
-// five rows are a quarter padding there.
-bool pair_sym_supported(int n) { return n >= 9 && n <= 20 && n != 11 && n != 12; }
+// error less than this kernel's; at 11 and 12 also, and three blocks of five rows are
+// a quarter padding there.  Below 16^3 sites (n = 16, a fifth padding: 8192) the
+// general kernel is the faster one: L = 8, n = 16, 1500 configurations 103 against 211
+// us, L = 12, n = 19, 24 of them 23 against 30; from there on this one: L = 16, n = 9,
+// one configuration 19 / 19, n = 19, 200 of them 175 against 111, L = 32, n = 10, 64
+// 126 against 80.
+bool pair_sym_supported(int n, long vol) {
+  return n >= 9 && n <= 20 && n != 11 && n != 12 && vol >= (n == 16 ? 8192 : 4096);
+}
 
 // flags: the device's check of the table (nonzero: the kernel writes
 // nothing), or null where the caller knows that the table qualifies.
