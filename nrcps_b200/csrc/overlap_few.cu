@@ -206,7 +206,8 @@ nrcps_status launch_few(nrcps_context* ctx, const float* src, int ns, const void
 // 15 against 22; but not those of very many configurations, which are a CTA each
 // at least (L = 8, N = 2, 1000 of them 32 against 21), nor of one to three sources
 // on many sites, where most of a block of five is padding (L = 48, N = 1, 100
-// configurations 98 against 61), nor, with more than five, large volumes, where
+// configurations 98 against 61), nor of one or two orbitals (L = 32, 10 sources, 200
+// configurations 114 against 52), nor, with more than five, large volumes, where
 // a cluster of eight per configuration leaves the chip empty (L = 48, N = 7, 16
 // configurations 122 against 73).  Large ones where the blocks of five are full
 // and a configuration has many tiles: L = 48, N = 10, 128 configurations 459
@@ -218,7 +219,9 @@ bool overlap_few_pays(int ns, int nt, int nconf, long vol) {
   const long l32 = 32 * 32 * 32, sites = nconf * vol;
   if ((double)nt * sites <= (double)(1 << 24)) {
     if (ns <= 3) return nconf <= 128 && sites <= 1 << 22;
-    return ns <= FB ? nconf <= 512 : nconf <= 320 && vol <= l32;
+    if (nt <= 2) return nconf <= 128 && sites < 1 << 21;
+    const long ctas = (long)nconf * ((nt + 2 * FB - 1) / (2 * FB));
+    return ns <= FB ? ctas <= 512 : ctas <= 320 && vol <= l32;
   }
   const long padded = (long)((ns + FB - 1) / FB) * ((nt + FB - 1) / FB) * FB * FB, full = (long)ns * nt;
   return (9 * padded <= 10 * full || (4 * padded <= 5 * full && nconf <= 128)) && vol >= l32 &&
