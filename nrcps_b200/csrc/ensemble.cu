@@ -22,7 +22,7 @@ nrcps_status slater_dets_dispatch(nrcps_context* ctx, const double* S, const dou
 size_t slater_dets_scratch_bytes(int N, int nconf, int mode);
 nrcps_status overlap_impl(nrcps_context* ctx, const double* src, int ns, const void* psi, int nt, int nconf,
                           long vol, nrcps_precision prec, double* S, double* part);
-size_t overlap_part_bytes(nrcps_context* ctx, int ns, int nt, int nconf, long vol);
+size_t overlap_part_bytes(nrcps_context* ctx, int ns, int nt, int nconf, long vol, nrcps_precision prec);
 nrcps_status gather_impl(nrcps_context* ctx, const int* index, int ns, const void* psi, int nt, int nconf, long vol,
                          nrcps_precision prec, double* S);
 nrcps_status pair_impl(nrcps_context* ctx, const void* psi1, const void* psi2, int n, int nconf, long vol,
@@ -280,7 +280,7 @@ extern "C" nrcps_status nrcps_ensemble_create(nrcps_context* ctx, const nrcps_jo
       if ((st = dalloc(ctx, (char**)&e->src_split, overlap_tc_split_bytes(N, V))) ||
           (st = overlap_tc_prepare(ctx, e->src, N, V, N, nc, e->src_split)))
         return fail(st);
-    } else if ((st = dalloc(ctx, (char**)&e->src_part, overlap_part_bytes(ctx, N, N, nc, V)))) {
+    } else if ((st = dalloc(ctx, (char**)&e->src_part, overlap_part_bytes(ctx, N, N, nc, V, (nrcps_precision)job->precision)))) {
       return fail(st);
     }
   }

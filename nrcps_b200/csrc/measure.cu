@@ -22,7 +22,7 @@ namespace cg = cooperative_groups;
 // eighth) one after the other; the groups one after the other.  Who does which
 // is free: one CTA all of a configuration, a cluster a group per CTA, or, where
 // few configurations leave the chip idle, a CTA a few chunks whose sums go to
-// `out` one by one and overlap_sum_kernel adds up.
+// `out` one by one and overlap_sum_kernel adds up; or overlap_direct_kernel.
 //
 // Why chunks: one configuration's overlap is 47 M FP64 FMAs at N = 19, L = 32,
 // 3 us of the whole chip, and the reference's drivers measure one
@@ -38,7 +38,7 @@ struct OvTile {
   int rows, T, lanes;
   int log_t;         // T = 1 << log_t
 };
-__host__ __device__ inline OvTile overlap_tiles(int ns, int nt) {
+static OvTile overlap_tiles(int ns, int nt) {
   OvTile o;
   const int bs = (ns + 3) / 4, bt = (nt + 3) / 4;
   if (bs * bt <= 32) {
@@ -49,30 +49,34 @@ __host__ __device__ inline OvTile overlap_tiles(int ns, int nt) {
   }
   o.ns_t = (bs + o.ts - 1) / o.ts, o.nt_t = (bt + o.tt - 1) / o.tt;
   o.rows = 4 * (o.ts + o.tt);
-  // both buffers of two CTAs fit an SM up to 48 rows
-  o.log_t = o.rows <= 8 ? 8 : o.rows <= 24 ? 7 : o.rows <= 48 ? 6 : 5;
-  o.T = 1 << o.log_t;
   o.lanes = 8;
   while (2 * o.lanes * o.ts * o.tt <= OV_THREADS && 2 * o.lanes <= 32) o.lanes *= 2;
   return o;
 }
 
-// Chunks of a configuration's sites and their groups.  512 sites: a chunk's tree
-// and its share of the sums cost about a tenth of its FMAs there; half as many in
-// small volumes, where a call waits for its longest CTA (N = 19, L = 8: 17 us, one
-// chunk of 512 25); at most 512 chunks (the sums' buffer).
+// Chunks of a configuration's sites and their groups.  A lane's sums run over 64
+// sites of a chunk (the tree and its share of the sums are then a tenth of the
+// FMAs), over fewer in small volumes: a call waits for its longest CTA there, and 256
+// threads a site apart, which were here before, had sums as short (a lane's
+// 32 sites at N = 19 and L = 8 would have 1.8 times the error, rms).  At most 512
+// chunks (the sums' buffer).
 constexpr int OV_GROUPS = 8;
 struct OvChunks {
   long sites;                       // of a chunk, a multiple of T
   int chunks, per_group, groups;
 };
-__host__ __device__ inline OvChunks overlap_chunks(long vol) {
+static OvChunks overlap_chunks(long vol, OvTile& o) {
   OvChunks c;
-  c.sites = vol <= 2048 ? 256 : 512;
+  c.sites = o.lanes * (vol <= 1024 ? 4 : vol <= 2048 ? 8 : vol <= 4096 ? 16 : vol <= 16384 ? 32 : 64);
+  if (c.sites > 512) c.sites = 512;
   while ((vol + c.sites - 1) / c.sites > 512) c.sites *= 2;
   c.chunks = (int)((vol + c.sites - 1) / c.sites);
   c.per_group = (c.chunks + OV_GROUPS - 1) / OV_GROUPS;
   c.groups = (c.chunks + c.per_group - 1) / c.per_group;
+  // stages: both buffers of two CTAs fit an SM up to 48 rows
+  o.log_t = o.rows <= 8 ? 8 : o.rows <= 24 ? 7 : o.rows <= 48 ? 6 : 5;
+  while ((1 << o.log_t) > c.sites) --o.log_t;
+  o.T = 1 << o.log_t;
   return c;
 }
 
@@ -265,38 +269,47 @@ __global__ void __launch_bounds__(OV_THREADS, 2) overlap_tile_kernel(const doubl
   cluster.sync();  // peers keep their shared memory until every sum is read
 }
 
-// The same sums for up to eight sources where an entry has 32 lanes, without
-// staging: a warp takes one orbital and one group of its chunks, SB sources in
-// registers; the groups of an orbital meet in shared memory.  With few sources
-// there is little to reuse, the orbitals are the traffic, and the tile kernel
-// keeps too few bytes in flight (a 4 x 4 block mostly padding on top): N = 2, FP64,
-// 1000 configurations at L = 48 688 us (5.1 TB/s) against 4.2 ms, 300 at L = 32
-// 85 against 407; a block per orbital: 1328 and 163.
+// The same sums without staging: LANES lanes take one orbital and one group of its
+// chunks, SB sources (of blockIdx.y's) in registers; the groups of an orbital meet
+// in shared memory.  With few sources or orbitals there is little to reuse, the
+// orbitals are the traffic, and the tile kernel keeps too few bytes in flight (a
+// 4 x 4 block mostly padding on top); in small calls its chain is the shorter one.
+// FP64, N = 2, 300 configurations at L = 32: 69 us against 407 by tiles (a block
+// per orbital: 163); 19 sources and one orbital, L = 16, 1500 configurations 150
+// against 510 (148); N = 19, L = 8, one configuration 12 (12).  Four sites in flight
+// per lane: with two N = 10, L = 16, 512 takes 483 us against 434, three CTAs of 80
+// registers spill.
 constexpr int OD_WARPS = 8;
-template <typename R, int SB>
+constexpr int overlap_direct_sources(int ns) { return ns <= 2 ? 2 : ns <= 4 ? 4 : 8; }
+template <typename R, int SB, int LANES>
 __global__ void __launch_bounds__(32 * OD_WARPS, SB == 8 ? 2 : 3)
     overlap_direct_kernel(const double2* __restrict__ src, int ns, const void* __restrict__ psi, int nt, long vol,
                           long orbitals, OvChunks ch, double* __restrict__ S) {
-  __shared__ double2 sums[OD_WARPS][SB];
-  const int l = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int here = OD_WARPS / ch.groups, g = warp % ch.groups;  // orbitals of this CTA, the warp's group
-  const long first = (long)blockIdx.x * here, orbital = first + warp / ch.groups;
+  constexpr int SUB = 32 / LANES;  // orbitals of a warp
+  __shared__ double2 sums[OD_WARPS][SUB][SB];
+  const int l = threadIdx.x % LANES, sub = threadIdx.x % 32 / LANES, warp = threadIdx.x >> 5;
+  const int s0 = SB * (int)blockIdx.y, sb = ns - s0 < SB ? ns - s0 : SB;
+  const double2* from = src + (size_t)s0 * vol;
+  const int here = OD_WARPS / ch.groups, g = warp % ch.groups;  // warps per group of this CTA, the warp's group
+  const long first = (long)blockIdx.x * here * SUB, orbital = first + warp / ch.groups * SUB + sub;
   const bool active = warp < here * ch.groups && orbital < orbitals;
   const cplx<R>* orb = reinterpret_cast<const cplx<R>*>(psi) + (size_t)(active ? orbital : 0) * vol;
   double gr = 0.0, gi = 0.0;
-  const int last = !active ? 0 : (g + 1) * ch.per_group < ch.chunks ? (g + 1) * ch.per_group : ch.chunks;
+  // (a warp's lanes go through the same chunks: the tree's shuffles are the warp's)
+  const int end_chunk = (g + 1) * ch.per_group < ch.chunks ? (g + 1) * ch.per_group : ch.chunks;
+  const int last = warp < here * ch.groups ? end_chunk : 0;
   for (int chunk = g * ch.per_group; chunk < last; ++chunk) {
     double re[SB], im[SB];
 #pragma unroll
     for (int k = 0; k < SB; ++k) re[k] = im[k] = 0.0;
     const long end = (chunk + 1) * ch.sites < vol ? (chunk + 1) * ch.sites : vol;
 #pragma unroll 4
-    for (long q = chunk * ch.sites + l; q < end; q += 32) {
+    for (long q = chunk * ch.sites + l; q < end; q += LANES) {
       const cplx<R> v = orb[q];
       const double br = (double)v.re, bi = (double)v.im;
       double2 a[SB];
 #pragma unroll
-      for (int u = 0; u < SB; ++u) a[u] = u < ns ? __ldg(src + (size_t)u * vol + q) : make_double2(0.0, 0.0);
+      for (int u = 0; u < SB; ++u) a[u] = u < sb ? __ldg(from + (size_t)u * vol + q) : make_double2(0.0, 0.0);
 #pragma unroll
       for (int u = 0; u < SB; ++u) {
         re[u] = fma(a[u].x, br, re[u]);
@@ -305,22 +318,23 @@ __global__ void __launch_bounds__(32 * OD_WARPS, SB == 8 ? 2 : 3)
         im[u] = fma(-a[u].y, br, im[u]);
       }
     }
-    overlap_tree<SB>(re, im, l, 32);
+    overlap_tree<SB>(re, im, l, LANES);
     gr += re[0];
     gi += im[0];
   }
-  if (l % (32 / SB) == 0) sums[warp][overlap_first<SB>(l, 32)] = make_double2(gr, gi);
+  if (l % (LANES / SB) == 0) sums[warp][sub][overlap_first<SB>(l, LANES)] = make_double2(gr, gi);
   __syncthreads();
-  for (int e = threadIdx.x; e < here * SB; e += 32 * OD_WARPS) {
-    const int s = e % SB, k = e / SB;
-    if (s >= ns || first + k >= orbitals) continue;
+  for (int e = threadIdx.x; e < here * SUB * SB; e += 32 * OD_WARPS) {
+    const int s = e % SB, k = e / SB;  // orbital first + k
+    if (s >= sb || first + k >= orbitals) continue;
     double2 v = make_double2(0.0, 0.0);
     for (int i = 0; i < ch.groups; ++i) {
-      v.x += sums[k * ch.groups + i][s].x;
-      v.y += sums[k * ch.groups + i][s].y;
+      const double2 w = sums[k / SUB * ch.groups + i][k % SUB][s];
+      v.x += w.x;
+      v.y += w.y;
     }
     const long conf = (first + k) / nt, t = (first + k) % nt;
-    double* to = S + 2 * ((conf * ns + s) * nt + t);
+    double* to = S + 2 * ((conf * ns + s0 + s) * nt + t);
     to[0] = v.x;
     to[1] = v.y;
   }
@@ -1348,46 +1362,72 @@ static OvSplit overlap_split(const nrcps_context* ctx, const OvTile& o, const Ov
   return {(int)((ch.chunks + per - 1) / per), (int)per, true};
 }
 
-// Where the kernel without staging is the faster one: a chunk per group at most
-// (up to L = 16), or orbitals enough to fill the chip.  It against the tile kernel,
-// FP64, us: N = 7, L = 16, 40 configurations 16 / 22; N = 7, L = 32, 4
-// configurations 40 / 23, 16 42 / 48; N = 4, L = 32, one 33 / 17, 40 70 / 89; N = 8,
-// L = 16, 300 93 / 106, 1000 282 / 256.
-static bool overlap_direct_pays(int ns, int nt, int nconf, bool fp64, const OvTile& o, const OvChunks& ch) {
-  if (o.lanes < 32 || ns > 8) return false;
-  const long orbitals = (long)nconf * nt;
-  if (fp64 && ns > 4 && orbitals > 4096) return false;
-  return ch.per_group == 1 || orbitals >= 10L * ns;
+// Whether the kernel without staging is the faster one, by what either takes in
+// microseconds beyond a launch.  It: rounds of CTAs times the sites of a lane, and
+// the loads and FMAs of every orbital with every group of sources; by tiles:
+// rounds times sites of a lane, the rows staged, CTAs, and the second kernel.
+// Fitted to both kernels over N = 1 .. 33, L = 8 .. 48, one to 4096 configurations
+// (1324 calls): the choice costs 1.5 % in the mean of what always taking the faster
+// one would.  In small volumes the sources stay in L1 while there are few orbitals.
+// What is left against a block per orbital of 256 threads, the kernel before: N = 5 to
+// 10 in batches of 10^5 to 10^7 sites, up to a third slower (N = 5, L = 12, 1500
+// configurations 159 against 120 us, N = 10, L = 12, 512 173 against 153).
+static bool overlap_direct_pays(const nrcps_context* ctx, int ns, int nt, int nconf, long vol, bool fp64, const OvTile& o,
+                                const OvChunks& ch, const OvSplit& split) {
+  const int sb = overlap_direct_sources(ns);
+  const double sources = (ns + sb - 1) / sb;
+  const long orbitals = (long)nconf * nt, here = OD_WARPS / ch.groups * (32 / o.lanes);
+  const double entries = (double)orbitals * vol;
+  const double slots = (sb == 8 ? 2.0 : 3.0) * ctx->sm_count;
+  double direct = 0.03 * ceil(((orbitals + here - 1) / here) * sources / slots) * ch.per_group * ch.sites / o.lanes * (sb + 1) +
+                  1e-6 * entries * sources * (0.15 * sb + 1.3);
+  if (vol <= 4096 && entries < 5e6) direct *= 0.85;
+  else if (vol <= 4096 && o.lanes < 32 && fp64) direct *= 1.25;
+  const double ctas = (double)nconf * o.ns_t * o.nt_t * split.ctas, sites = (double)split.per_cta * ch.sites;
+  const double tiles = 1.0 + (split.each ? 3.7 : 0.0) + 0.2 * ceil(ctas / (2.0 * ctx->sm_count)) * sites / o.lanes +
+                       3e-6 * ctas * sites * o.rows + 5e-3 * ctas;
+  return direct < tiles;
 }
 
 // What an ensemble of these overlaps brings for the sums (0: nothing).
-size_t overlap_part_bytes(nrcps_context* ctx, int ns, int nt, int nconf, long vol) {
-  const OvTile o = overlap_tiles(ns, nt);
-  const OvChunks ch = overlap_chunks(vol);
-  return overlap_split(ctx, o, ch, ns, nt, nconf, true).each ? sizeof(double2) * (size_t)nconf * ns * nt * ch.chunks : 0;
+size_t overlap_part_bytes(nrcps_context* ctx, int ns, int nt, int nconf, long vol, nrcps_precision prec) {
+  OvTile o = overlap_tiles(ns, nt);
+  const OvChunks ch = overlap_chunks(vol, o);
+  const OvSplit split = overlap_split(ctx, o, ch, ns, nt, nconf, true);
+  if (!split.each || overlap_direct_pays(ctx, ns, nt, nconf, vol, prec == NRCPS_F64, o, ch, split)) return 0;
+  return sizeof(double2) * (size_t)nconf * ns * nt * ch.chunks;
 }
 
 template <typename R>
 static nrcps_status launch_overlap(nrcps_context* ctx, const double* src, int ns, const void* psi, int nt, int nconf,
                                    long vol, double* S, double* part) {
-  const OvTile o = overlap_tiles(ns, nt);
-  const OvChunks ch = overlap_chunks(vol);
-  if (overlap_direct_pays(ns, nt, nconf, sizeof(R) == 8, o, ch)) {
-    const long orbitals = (long)nconf * nt, here = OD_WARPS / ch.groups;
+  OvTile o = overlap_tiles(ns, nt);
+  const OvChunks ch = overlap_chunks(vol, o);
+  OvSplit split = overlap_split(ctx, o, ch, ns, nt, nconf, true);
+  if (overlap_direct_pays(ctx, ns, nt, nconf, vol, sizeof(R) == 8, o, ch, split)) {
+    const long orbitals = (long)nconf * nt, here = OD_WARPS / ch.groups * (32 / o.lanes);
+    const int sb = overlap_direct_sources(ns);
     auto launch = [&](auto kern) {
-      kern<<<(unsigned)((orbitals + here - 1) / here), 32 * OD_WARPS, 0, ctx->stream>>>(
-          reinterpret_cast<const double2*>(src), ns, psi, nt, vol, orbitals, ch, S);
+      kern<<<dim3((unsigned)((orbitals + here - 1) / here), (unsigned)((ns + sb - 1) / sb)), 32 * OD_WARPS, 0,
+             ctx->stream>>>(reinterpret_cast<const double2*>(src), ns, psi, nt, vol, orbitals, ch, S);
     };
-    if (ns <= 2) launch(overlap_direct_kernel<R, 2>);
-    else if (ns <= 4) launch(overlap_direct_kernel<R, 4>);
-    else launch(overlap_direct_kernel<R, 8>);
+    switch (100 * sb + o.lanes) {
+      case 208: launch(overlap_direct_kernel<R, 2, 8>); break;
+      case 216: launch(overlap_direct_kernel<R, 2, 16>); break;
+      case 232: launch(overlap_direct_kernel<R, 2, 32>); break;
+      case 408: launch(overlap_direct_kernel<R, 4, 8>); break;
+      case 416: launch(overlap_direct_kernel<R, 4, 16>); break;
+      case 432: launch(overlap_direct_kernel<R, 4, 32>); break;
+      case 808: launch(overlap_direct_kernel<R, 8, 8>); break;
+      case 816: launch(overlap_direct_kernel<R, 8, 16>); break;
+      default: launch(overlap_direct_kernel<R, 8, 32>);
+    }
     ctx->launches++;
     return check_launch(ctx, "overlap_direct_kernel");
   }
   const size_t smem = sizeof(double2) * (2 * (size_t)o.rows * o.T + 2 * 16 * o.ts * o.tt);
   // (132 rows of 32 sites and 32 blocks are the most)
   NRCPS_TRY(allow_smem(ctx, (const void*)overlap_tile_kernel<R>, 160 * 1024, "overlap_tile: smem attribute"));
-  OvSplit split = overlap_split(ctx, o, ch, ns, nt, nconf, true);
   bool shared = false;
   if (split.each && !part) {
     part = overlap_context_part(ctx);
