@@ -104,9 +104,11 @@ const char *nrcps_version(void);
  *                      st.async onto the owner CTA's mbarrier (one cluster
  *                      barrier per orbital);
  *   "overlap.tc"       1 (default): dense-source overlaps of FP32 orbitals
- *                      on the tcgen05 tensor cores (TF32 hi/lo split, FP32
- *                      accumulation) where V is a multiple of 16; 0: the
- *                      CUDA-core kernel with FP64 accumulation;
+ *                      where V is a multiple of 16 on the tcgen05 tensor
+ *                      cores (TF32 hi/lo split, FP32 accumulation), with up
+ *                      to ten sources on the CUDA cores (FP32 sources, FP32
+ *                      accumulation) where that is faster; 0: the CUDA-core
+ *                      kernel with FP64 accumulation;
  *   "fused.zpos"       1 (default): for a Z2 field with a position factor the
  *                      fused step reads both weights of every site,
  *                      (1 +- a) P(x)/V, from a table made ahead of the step;
@@ -129,8 +131,10 @@ const char *nrcps_version(void);
  *                      stream windows, the same results); 0: each run draws
  *                      its own fields before its graph;
  *   "lu.warp"          1 (default): leading-minor determinants with one warp
- *                      per minor in shared memory (N <= 64); 0: one thread
- *                      per minor with global scratch;
+ *                      or a segment of one per minor, its rows in registers
+ *                      (N <= 32) or the minor in shared memory (N <= 64, or
+ *                      matrices that do not start on 16 bytes); 0: one
+ *                      thread per minor with global scratch;
  *   "fused.wait_ns"    time limit of every mbarrier wait in the fused step,
  *                      in nanoseconds (default 2e9, minimum 1000).  A wait
  *                      that runs out sets the context's time-out flag and
@@ -138,7 +142,10 @@ const char *nrcps_version(void);
  *                      nrcps_synchronize returns NRCPS_ERR_TIMEOUT;
  *   "fused.stall_test" 1: the first wait of one CTA of the next fused steps
  *                      is made on an mbarrier nothing arrives on, so that it
- *                      runs out (a test of the time-out path); 0 (default). */
+ *                      runs out (a test of the time-out path); 0 (default).
+ *                      The kernels that hold an orbital in one SM or CTA
+ *                      (kinds 13 and 14 of nrcps_fused_choice) wait on no
+ *                      mbarrier: force a variant to test it there. */
 nrcps_status nrcps_set_option(nrcps_context *ctx, const char *name, long value);
 /* Times every fused-kernel variant (cluster size, lane split) for (prec, L)
  * on this device and keeps the fastest for later calls; *cluster receives
@@ -288,7 +295,11 @@ nrcps_status nrcps_propagate(nrcps_context *ctx, void *psi, int batch, int nconf
  * (src/one_body/noarch/one_body_project.C:14-27) and Cuda::InnerProduct
  * (src/utils/cuda/cuda_utils.cu:88-127): S[c][s][t] = sum_p conj(src_s(p))
  * psi_{c,t}(p), for nconf configurations; src (ns x V, FP64 complex) shared,
- * psi (nconf x nt x V, precision prec), S FP64 complex, row-major per conf. */
+ * psi (nconf x nt x V, precision prec), S FP64 complex, row-major per conf.
+ * FP64 orbitals: the order of the sums follows (ns, nt, V), so a
+ * configuration's S has the same bits in every batch.  FP32 orbitals (but for
+ * "overlap.tc" 0): kernel and split follow nconf too, and S may differ between
+ * batches by the kernels' rounding, some 1e-6 of the largest |S|. */
 nrcps_status nrcps_overlap(nrcps_context *ctx, const double *dev_src, int ns, const void *dev_psi,
                            int nt, int nconf, long vol, nrcps_precision prec, double *dev_S);
 /* Plane-wave sources (OneBody::Set(n1,n2,n3), src/one_body/one_body.C:215-228):

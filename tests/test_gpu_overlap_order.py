@@ -1,5 +1,5 @@
 """The CUDA-core overlap's order of summation: given by the shape, not by the
-batch, the buffer at hand or a capture."""
+batch, the buffer at hand or a capture; what FP32 orbitals may differ by."""
 import pytest
 import torch
 
@@ -52,3 +52,22 @@ def test_very_many_orbitals(precision, nt, vol):
     want = torch.einsum("sv,ctv->cst", src.conj(), p)
     size = torch.einsum("sv,ctv->cst", src.abs(), p.abs())
     assert ((got - want).abs() <= (1e-14 if precision == "f64" else 3e-6) * size).all()
+
+
+@pytest.mark.parametrize("n,vol,batch", [(10, 13824, 130), (7, 4096, 700), (10, 4096, 5), (4, 32768, 40)])
+def test_fp32_alone_and_in_a_batch(n, vol, batch):
+    """FP32 orbitals and up to ten sources: kernel and split follow the batch.
+    The tensor-core kernel is held to 1e-6 of the largest |S|, the packed one
+    to 56 x 2^-24 of the sum of moduli (39 roundings a real part): a
+    configuration alone and in a batch are within the two of each other."""
+    import nrcps_b200 as nb
+    ctx = nb.default_context()
+    g = torch.Generator(device=ctx.device).manual_seed(n * 1000 + batch)
+    src = torch.randn((n, vol), dtype=torch.complex128, device=ctx.device, generator=g)
+    psi = torch.randn((batch, n, vol), dtype=torch.complex64, device=ctx.device, generator=g)
+    got = nb.overlap(src, psi, ctx)
+    for c in (0, batch - 1):
+        alone = nb.overlap(src, psi[c:c + 1], ctx)[0]
+        size = src.abs() @ psi[c].to(torch.complex128).abs().T
+        bound = 1e-6 * alone.abs().max() + 56 * 2.0 ** -24 * size
+        assert ((got[c] - alone).abs() <= bound).all()
