@@ -246,6 +246,9 @@ NCU_TRAFFIC_PER_ORBITAL = {
     ("f32", 32, 11, 8): ((640.81e6 + 577.95e6) / 2432,
                          "ncu, kind 11 cluster 8, 2432 orbitals: 640.8 MB read + 577.9 MB written, scaled by orbitals "
                          "(profiles/fused_step_async_L32_f32.md)"),
+    ("f32", 32, 13, 1): ((899.68e6 + 564.04e6) / 2368,
+                         "ncu, kind 13, 2368 orbitals: 899.7 MB read + 564.0 MB written, scaled by orbitals "
+                         "(profiles/whole_orbital_steps_and_measurements.md)"),
     ("f32", 48, 11, 12): ((898.52e6 + 840.19e6) / 1007,
                           "ncu, kind 11 cluster 12, 1007 orbitals: 898.5 MB read + 840.2 MB written, scaled by "
                           "orbitals (profiles/fused_step_async_L48_f32_trapped.md)"),
@@ -256,6 +259,8 @@ NCU_PIPES = {
                         "source": "profiles/fused_step_L32_f32.md"},
     ("f32", 32, 11, 8): {"fma_pipe_pct": 41.7, "issue_active_pct": 51.3, "warps_per_sm": 15.0,
                          "source": "profiles/fused_step_async_L32_f32.md"},
+    ("f32", 32, 13, 1): {"fma_pipe_pct": 49.4, "issue_active_pct": 58.0, "warps_per_sm": 16.0,
+                         "source": "profiles/whole_orbital_steps_and_measurements.md"},
     ("f32", 48, 11, 12): {"fma_pipe_pct": 36.8, "issue_active_pct": 43.3, "warps_per_sm": 11.3,
                           "source": "profiles/fused_step_async_L48_f32_trapped.md"},
 }
@@ -458,7 +463,7 @@ def trapped_core(ctx, n_conf: int, steps: int, warmup: int, cpu_slices: int, pre
            "config": {"workload": f"trapped few-body L={L}^3 T={T}, SHO N={N}+{N} (lambda 4), [K,V,I,V,K] harmonic "
                                   f"EXP trap kappa={TRAPPED['kappa']}, Z2 a=0.5 RANLXS2 seed {TRAPPED['seed']}, "
                                   f"SlaterDet2 on the TGND pair sink, {n_conf} configs/step, FP32 propagation, "
-                                  f"TF32-split tensor-core overlap, FP64 LU, QR every 8",
+                                  f"FP32 overlap summed in FP64, FP64 LU, QR every 8",
                       "configs_per_step": n_conf, "l2": "orbitals %.1f GB (larger than L2)" % (n_conf * N * V * 8 / 1e9)},
            "e2e": {"value": n_conf * T / (e2e_ms / 1000.0), "unit": UNIT,
                    "h2d_bytes_per_step": src_host.numel() * 16, "d2h_bytes_per_step": dets_host.numel() * 16},
@@ -473,7 +478,8 @@ def trapped_core(ctx, n_conf: int, steps: int, warmup: int, cpu_slices: int, pre
                         "fp32": {"convention": "10 V log2 V flops per orbital-step",
                                  "achieved_tflops": round(fp32_tflops, 2), "peak_tflops": round(fp32_peak, 1),
                                  "frac": round(fp32_tflops / fp32_peak, 4)}},
-           "overlap": {"kernel": "tcgen05 TF32 hi/lo overlap S = src^H psi (incl. the source split)",
+           "overlap": {"kernel": "nrcps_overlap S = src^H psi, ten sources: packed FP32 on the CUDA cores from 32 configs "
+                                 "on, else tcgen05 TF32 hi/lo (incl. rounding the sources)",
                        "ms": round(oms, 3), "achieved_gbs": round(read_bytes / (oms / 1000) / 1e9, 1),
                        "frac_hbm": round(read_bytes / (oms / 1000) / 1e9 / peak, 4),
                        "useful_tflops": round(overlap_flops / (oms / 1000) / 1e12, 2)},

@@ -57,8 +57,8 @@ static OvTile overlap_tiles(int ns, int nt) {
 // Chunks of a configuration's sites and their groups.  A lane's sums run over 64
 // sites of a chunk (the tree and its share of the sums are then a tenth of the
 // FMAs), over fewer in small volumes: a call waits for its longest CTA there, and 256
-// threads a site apart, which were here before, had sums as short (a lane's
-// 32 sites at N = 19 and L = 8 would have 1.8 times the error, rms).  At most 512
+// threads a site apart, which were here before, had sums as short (32 of a
+// lane's at N = 19 and L = 8 would have 1.7 times the error, rms).  At most 512
 // chunks (the sums' buffer).
 constexpr int OV_GROUPS = 8;
 struct OvChunks {
@@ -274,11 +274,11 @@ __global__ void __launch_bounds__(OV_THREADS, 2) overlap_tile_kernel(const doubl
 // in shared memory.  With few sources or orbitals there is little to reuse, the
 // orbitals are the traffic, and the tile kernel keeps too few bytes in flight (a
 // 4 x 4 block mostly padding on top); in small calls its chain is the shorter one.
-// FP64, N = 2, 300 configurations at L = 32: 69 us against 407 by tiles (a block
-// per orbital: 163); 19 sources and one orbital, L = 16, 1500 configurations 150
-// against 510 (148); N = 19, L = 8, one configuration 12 (12).  Four sites in flight
-// per lane: with two N = 10, L = 16, 512 takes 483 us against 434, three CTAs of 80
-// registers spill.
+// FP64, N = 2, 200 configurations at L = 32: 47 us against 285 by tiles (a block
+// per orbital: 87); 19 sources and one orbital, L = 16, 1500 configurations 150
+// against 510 (148); N = 9, L = 8, one configuration 12 against 17 (12).  Four sites
+// in flight per lane: two cost 13 % in the mean over N = 1 .. 33, L = 8 .. 48, one
+// with three CTAs of 80 registers 32 %.
 constexpr int OD_WARPS = 8;
 constexpr int overlap_direct_sources(int ns) { return ns <= 2 ? 2 : ns <= 4 ? 4 : 8; }
 template <typename R, int SB, int LANES>
