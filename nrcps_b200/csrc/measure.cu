@@ -3,6 +3,7 @@
 // FP64 LU of every leading minor with the reference's pivoting rule.
 #include <cooperative_groups.h>
 
+#include <type_traits>
 #include "common.cuh"
 
 namespace nrcps {
@@ -270,25 +271,32 @@ __global__ void __launch_bounds__(OV_THREADS, 2) overlap_tile_kernel(const doubl
 }
 
 // The same sums without staging: LANES lanes take one orbital and one group of its
-// chunks, SB sources (of blockIdx.y's) in registers; the groups of an orbital meet
+// chunks, NX sources (blockIdx.y's) in registers; the groups of an orbital meet
 // in shared memory.  With few sources or orbitals there is little to reuse, the
 // orbitals are the traffic, and the tile kernel keeps too few bytes in flight (a
 // 4 x 4 block mostly padding on top); in small calls its chain is the shorter one.
 // FP64, N = 2, 200 configurations at L = 32: 47 us against 285 by tiles (a block
 // per orbital: 87); 19 sources and one orbital, L = 16, 1500 configurations 150
 // against 510 (148); N = 9, L = 8, one configuration 12 against 17 (12).  Four sites
-// in flight per lane: two cost 13 % in the mean over N = 1 .. 33, L = 8 .. 48, one
-// with three CTAs of 80 registers 32 %.
+// in flight per lane: two cost 13 % in the mean over N = 1 .. 33, L = 8 .. 48.  As many
+// sources as there are: groups of eight with the rest masked took 7 % more (N = 10,
+// L = 12, 512 configurations 210 us, now 146).
 constexpr int OD_WARPS = 8;
-constexpr int overlap_direct_sources(int ns) { return ns <= 2 ? 2 : ns <= 4 ? 4 : 8; }
-template <typename R, int SB, int LANES>
-__global__ void __launch_bounds__(32 * OD_WARPS, SB == 8 ? 2 : 3)
+
+// Sources of a group: near-equal groups of at most eight
+constexpr int overlap_direct_sources(int ns) {
+  return ns <= 2 ? 2 : ns <= 4 ? 4 : (ns + (ns + 7) / 8 - 1) / ((ns + 7) / 8);
+}
+
+template <typename R, int NX, int LANES, bool MANY>
+__global__ void __launch_bounds__(32 * OD_WARPS, NX <= 4 || MANY ? 3 : 2)
     overlap_direct_kernel(const double2* __restrict__ src, int ns, const void* __restrict__ psi, int nt, long vol,
                           long orbitals, OvChunks ch, double* __restrict__ S) {
-  constexpr int SUB = 32 / LANES;  // orbitals of a warp
+  constexpr int SUB = 32 / LANES, SB = NX <= 2 ? 2 : NX <= 4 ? 4 : 8;  // orbitals of a warp, entries of the tree
+  constexpr int UNROLL = MANY ? 2 : 4;
   __shared__ double2 sums[OD_WARPS][SUB][SB];
   const int l = threadIdx.x % LANES, sub = threadIdx.x % 32 / LANES, warp = threadIdx.x >> 5;
-  const int s0 = SB * (int)blockIdx.y, sb = ns - s0 < SB ? ns - s0 : SB;
+  const int s0 = NX * (int)blockIdx.y, sb = ns - s0 < NX ? ns - s0 : NX;
   const double2* from = src + (size_t)s0 * vol;
   const int here = OD_WARPS / ch.groups, g = warp % ch.groups;  // warps per group of this CTA, the warp's group
   const long first = (long)blockIdx.x * here * SUB, orbital = first + warp / ch.groups * SUB + sub;
@@ -303,15 +311,15 @@ __global__ void __launch_bounds__(32 * OD_WARPS, SB == 8 ? 2 : 3)
 #pragma unroll
     for (int k = 0; k < SB; ++k) re[k] = im[k] = 0.0;
     const long end = (chunk + 1) * ch.sites < vol ? (chunk + 1) * ch.sites : vol;
-#pragma unroll 4
+#pragma unroll UNROLL
     for (long q = chunk * ch.sites + l; q < end; q += LANES) {
       const cplx<R> v = orb[q];
       const double br = (double)v.re, bi = (double)v.im;
-      double2 a[SB];
+      double2 a[NX];
 #pragma unroll
-      for (int u = 0; u < SB; ++u) a[u] = u < sb ? __ldg(from + (size_t)u * vol + q) : make_double2(0.0, 0.0);
+      for (int u = 0; u < NX; ++u) a[u] = u < sb ? __ldg(from + (size_t)u * vol + q) : make_double2(0.0, 0.0);
 #pragma unroll
-      for (int u = 0; u < SB; ++u) {
+      for (int u = 0; u < NX; ++u) {
         re[u] = fma(a[u].x, br, re[u]);
         im[u] = fma(a[u].x, bi, im[u]);
         re[u] = fma(a[u].y, bi, re[u]);
@@ -1362,27 +1370,42 @@ static OvSplit overlap_split(const nrcps_context* ctx, const OvTile& o, const Ov
   return {(int)((ch.chunks + per - 1) / per), (int)per, true};
 }
 
+static long overlap_direct_ctas(int ns, int nt, int nconf, const OvTile& o, const OvChunks& ch) {
+  const long here = OD_WARPS / ch.groups * (32 / o.lanes), sb = overlap_direct_sources(ns);
+  return ((long)nconf * nt + here - 1) / here * ((ns + sb - 1) / sb);
+}
+
+// Groups of five or six sources, many CTAs: three per SM, two sites in flight (N = 5,
+// L = 12, 1500 configurations 113 us against 128 with two CTAs and four sites, N = 10,
+// L = 16, one 17 against 12).
+static bool overlap_direct_many(const nrcps_context* ctx, int ns, int nt, int nconf, const OvTile& o,
+                                const OvChunks& ch) {
+  const int sb = overlap_direct_sources(ns);
+  return (sb == 5 || sb == 6) && overlap_direct_ctas(ns, nt, nconf, o, ch) >= 8L * ctx->sm_count;
+}
+
 // Whether the kernel without staging is the faster one, by what either takes in
 // microseconds beyond a launch.  It: rounds of CTAs times the sites of a lane, and
 // the loads and FMAs of every orbital with every group of sources; by tiles:
 // rounds times sites of a lane, the rows staged, CTAs, and the second kernel.
 // Fitted to both kernels over N = 1 .. 33, L = 8 .. 48, one to 4096 configurations
-// (1324 calls): the choice costs 1.5 % in the mean of what always taking the faster
-// one would.  In small volumes the sources stay in L1 while there are few orbitals.
-// What is left against a block per orbital of 256 threads, the kernel before: N = 5 to
-// 10 in batches of 10^5 to 10^7 sites, up to a third slower (N = 5, L = 12, 1500
-// configurations 159 against 120 us, N = 10, L = 12, 512 173 against 153).
+// (1324 calls): the choice costs 1 % in the mean of what always taking the faster
+// one would.  In small volumes the sources stay in L1 while there are few orbitals;
+// eight accumulators in large batches there, and FP32 orbitals in large batches
+// elsewhere, take longer than the sum says.
+// What is left against a block per orbital of 256 threads, the kernel before: N = 7, 8
+// and 13 in batches of 10^5 to 10^6 sites, and one orbital of 4096 configurations, by
+// up to a third (N = 7, L = 12, 512 configurations 75 against 64 us).
 static bool overlap_direct_pays(const nrcps_context* ctx, int ns, int nt, int nconf, long vol, bool fp64, const OvTile& o,
                                 const OvChunks& ch, const OvSplit& split) {
   const int sb = overlap_direct_sources(ns);
-  const double sources = (ns + sb - 1) / sb;
-  const long orbitals = (long)nconf * nt, here = OD_WARPS / ch.groups * (32 / o.lanes);
-  const double entries = (double)orbitals * vol;
-  const double slots = (sb == 8 ? 2.0 : 3.0) * ctx->sm_count;
-  double direct = 0.03 * ceil(((orbitals + here - 1) / here) * sources / slots) * ch.per_group * ch.sites / o.lanes * (sb + 1) +
-                  1e-6 * entries * sources * (0.15 * sb + 1.3);
+  const double entries = (double)nconf * nt * vol;
+  const double slots = (sb <= 4 || overlap_direct_many(ctx, ns, nt, nconf, o, ch) ? 3.0 : 2.0) * ctx->sm_count;
+  double direct = 0.03 * ceil(overlap_direct_ctas(ns, nt, nconf, o, ch) / slots) * ch.per_group * ch.sites / o.lanes * (sb + 1) +
+                  1e-6 * entries * (0.2 * ns + 1.3 * ((ns + sb - 1) / sb));
   if (vol <= 4096 && entries < 5e6) direct *= 0.85;
-  else if (vol <= 4096 && o.lanes < 32 && fp64) direct *= 1.25;
+  else if (vol <= 4096 && sb >= 7 && o.lanes < 32 && fp64) direct *= 1.15;
+  else if (vol > 4096 && entries >= 2e7 && !fp64) direct *= 1.6;
   const double ctas = (double)nconf * o.ns_t * o.nt_t * split.ctas, sites = (double)split.per_cta * ch.sites;
   const double tiles = 1.0 + (split.each ? 3.7 : 0.0) + 0.2 * ceil(ctas / (2.0 * ctx->sm_count)) * sites / o.lanes +
                        3e-6 * ctas * sites * o.rows + 5e-3 * ctas;
@@ -1411,17 +1434,23 @@ static nrcps_status launch_overlap(nrcps_context* ctx, const double* src, int ns
       kern<<<dim3((unsigned)((orbitals + here - 1) / here), (unsigned)((ns + sb - 1) / sb)), 32 * OD_WARPS, 0,
              ctx->stream>>>(reinterpret_cast<const double2*>(src), ns, psi, nt, vol, orbitals, ch, S);
     };
-    switch (100 * sb + o.lanes) {
-      case 208: launch(overlap_direct_kernel<R, 2, 8>); break;
-      case 216: launch(overlap_direct_kernel<R, 2, 16>); break;
-      case 232: launch(overlap_direct_kernel<R, 2, 32>); break;
-      case 408: launch(overlap_direct_kernel<R, 4, 8>); break;
-      case 416: launch(overlap_direct_kernel<R, 4, 16>); break;
-      case 432: launch(overlap_direct_kernel<R, 4, 32>); break;
-      case 808: launch(overlap_direct_kernel<R, 8, 8>); break;
-      case 816: launch(overlap_direct_kernel<R, 8, 16>); break;
-      default: launch(overlap_direct_kernel<R, 8, 32>);
-    }
+    const bool many = overlap_direct_many(ctx, ns, nt, nconf, o, ch);
+    auto lanes = [&](auto l) {
+      constexpr int LANES = decltype(l)::value;
+      switch (2 * sb + many) {
+        case 4: return launch(overlap_direct_kernel<R, 2, LANES, false>);
+        case 8: return launch(overlap_direct_kernel<R, 4, LANES, false>);
+        case 10: return launch(overlap_direct_kernel<R, 5, LANES, false>);
+        case 11: return launch(overlap_direct_kernel<R, 5, LANES, true>);
+        case 12: return launch(overlap_direct_kernel<R, 6, LANES, false>);
+        case 13: return launch(overlap_direct_kernel<R, 6, LANES, true>);
+        case 14: return launch(overlap_direct_kernel<R, 7, LANES, false>);
+        default: return launch(overlap_direct_kernel<R, 8, LANES, false>);
+      }
+    };
+    if (o.lanes == 8) lanes(std::integral_constant<int, 8>());
+    else if (o.lanes == 16) lanes(std::integral_constant<int, 16>());
+    else lanes(std::integral_constant<int, 32>());
     ctx->launches++;
     return check_launch(ctx, "overlap_direct_kernel");
   }
